@@ -24,6 +24,8 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-Xcompiler", "-fPIC",
     "-shared",
+    # the optimiser takes the translation unit's kernels in parallel
+    "-split-compile", "0",
 ]
 
 
