@@ -2062,7 +2062,7 @@ class Batch : public BatchBase {
     fl.bounds = nullptr;
     fl.wait_polls = wait_polls_;
     fl.queue = queue_;
-    constexpr size_t smem = lean_smem_bytes<3, PT, NORMAL>();
+    constexpr size_t smem = lean_smem_bytes<3, PT, NT * PPT>();
     auto kern = k_g2p2g_lean<3, PT, NT, PPT, NORMAL, SINGLE, MAT>;
     int& per_sm =
         lean_per_sm_[(PPT == 2 ? 16 : 0) + (NT == 128 ? 8 : 0) + (NORMAL ? 4 : 0) + (SINGLE ? 2 : 0) + (MAT == 0 ? 1 : 0)];

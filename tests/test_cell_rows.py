@@ -1,0 +1,93 @@
+"""The point-per-thread kernel's per-cell nodal sums at the sizes where they
+can go wrong, against the oracle: items of one point, of a full and an
+overfull bin, cells of many points, windows that are wide along every axis,
+points that drift out of their item's tile, corners on the upper face of the
+domain and point-sampled maps. Tolerances are the forms' own: 1e-10 per field
+and step in FP64 (summation order only), 1e-4 in the mixed form."""
+import numpy as np
+import pytest
+
+import bridge
+from mpm_3d_b200 import inputs
+from mpm_3d_b200.native import GPUExplicitUSL
+from util import FP64_TOL, assert_close, field_floor
+
+pytestmark = pytest.mark.gpu
+
+N = 16
+H = 1.0 / N
+
+
+@pytest.fixture(scope="module", autouse=True)
+def restated_lib():
+    bridge.build_restated()
+
+
+def _cloud(x, v=(0.0, 0.0, 0.0), spin=2.0, E=1e4, dt=1e-4):
+    """A body of the given positions with a velocity gradient, on an N^3 grid."""
+    x = np.asarray(x, np.float64)
+    n = x.shape[0]
+    vol = (H / 2) ** 3
+    xt = np.asarray(v) + (x - x.mean(0)) @ (spin * np.array([[0.3, -1.0, 0.2], [1.0, -0.2, 0.5], [-0.4, 0.1, 0.6]]))
+    body = inputs.Body("cloud", np.full(n, 1000.0 * vol), np.full(n, vol), x, xt, np.ones(n, np.int32), E=E)
+    return inputs.Case("cloud", 3, (1.0,) * 3, (N,) * 3, dt, 8, [body])
+
+
+def _random(n, lo, hi, seed):
+    return np.random.default_rng(seed).uniform(np.asarray(lo) * H, np.asarray(hi) * H, (n, 3))
+
+
+def _faces():
+    """Points whose upper corner lies on the domain's upper face, whose
+    corners leave the domain (point-sampled), and ordinary ones beside them."""
+    a = 0.25 * np.cbrt((H / 2) ** 3)   # half the extent
+    x = _random(60, (12.3, 12.3, 12.3), (15.6, 15.6, 15.6), 5)
+    x[:10, 0] = 1.0 - a
+    x[10:20, 2] = 1.0 - 0.3 * a
+    x[20:30, 1] = 1.0 - 0.1 * H * 0.3
+    return x
+
+
+CLOUDS = {
+    "one_point": lambda: _cloud([[4.4 * H, 5.3 * H, 6.7 * H]], spin=0.0),
+    "two_bins_33": lambda: _cloud(_random(33, (3.2, 4.1, 4.1), (4.9, 7.9, 7.9), 1)),
+    "full_bin_512": lambda: _cloud(_random(512, (4.2, 4.2, 4.2), (7.8, 7.8, 7.8), 2)),
+    "overfull_bin_1025": lambda: _cloud(_random(1025, (4.2, 4.2, 4.2), (7.8, 7.8, 7.8), 3)),
+    "one_cell_300": lambda: _cloud(_random(300, (5.2, 5.2, 5.2), (5.8, 5.8, 5.8), 4)),
+    "all_wide": lambda: _cloud(np.round(_random(200, (3.6, 3.6, 3.6), (9.4, 9.4, 9.4), 6) / H) * H + 0.01 * H),
+    "faces": lambda: _cloud(_faces(), spin=0.5),
+    "drift": lambda: _cloud(_random(400, (3.1, 3.1, 3.1), (6.9, 6.9, 6.9), 7), v=(0.45 * H / 1e-4, 0.3 * H / 1e-4, 0.0)),
+    "drift_down": lambda: _cloud(_random(400, (8.1, 8.1, 8.1), (11.9, 11.9, 11.9), 8),
+                                 v=(0.0, -0.4 * H / 1e-4, -0.4 * H / 1e-4)),
+}
+
+
+@pytest.mark.parametrize("cap", [128, 256, 512])
+@pytest.mark.parametrize("name", sorted(CLOUDS))
+def test_cell_sums(name, cap):
+    case = CLOUDS[name]()
+    gpu = GPUExplicitUSL(case, keep_debug=True, kernel=("point_per_thread", cap))
+    ref = bridge.RestatedJob(case)
+    for s in range(6):
+        gpu.step(1)
+        ref.step(1)
+        for f in ("x", "x_t", "T", "v"):
+            assert_close(gpu.points(0, f), ref.points(0, f), FP64_TOL, f"{name} step {s} {f}", field_floor(case, f))
+        assert_close(gpu.nodes(0, "m"), ref.nodes(0, "m"), FP64_TOL, f"{name} step {s} nodal m")
+    gpu.synchronize()
+    gpu.close()
+
+
+# "faces" places corners exactly on the upper face, where the map is
+# discontinuous; the mixed form's extent is an FP32 number, so its corners lie
+# on either side of the face and the oracle does not apply
+@pytest.mark.parametrize("name", sorted(set(CLOUDS) - {"faces"}))
+def test_cell_sums_mixed(name):
+    case = CLOUDS[name]()
+    gpu = GPUExplicitUSL(case, mode="mixed")
+    ref = bridge.RestatedJob(case)
+    gpu.step(6)
+    ref.step(6)
+    for f in ("x", "x_t", "T"):
+        assert_close(gpu.points(0, f), ref.points(0, f), 1e-4, f"{name} {f}", field_floor(case, f))
+    gpu.close()
