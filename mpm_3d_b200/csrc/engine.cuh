@@ -21,6 +21,7 @@
 #pragma once
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -437,6 +438,8 @@ class Batch : public BatchBase {
     pinned_give(frame_stage_, frame_cap_);
     if (frame_dev_) cudaFree(frame_dev_);
     if (frame_ev_) cudaEventDestroy(frame_ev_);
+    for (cudaEvent_t e : dl_ev_)
+      if (e) cudaEventDestroy(e);
     if (upload_ev_) cudaEventDestroy(upload_ev_);
     if (fork_ev_) cudaEventDestroy(fork_ev_);
     for (int i = 0; i < kSideStreams; i++) {
@@ -671,11 +674,7 @@ class Batch : public BatchBase {
     MPM_CUDA_TRY(cudaStreamSynchronize(stream_));
     int flag = 0;
     MPM_CUDA_TRY(cudaMemcpy(&flag, err_, sizeof(int), cudaMemcpyDeviceToHost));
-    if (flag & kErrWideSpan) return fail(MPMGPU_ERR_DEVICE, "point corners span more than two cells (extent > cell size)");
-    if (flag & kErrElemAlias) return fail(MPMGPU_ERR_DEVICE, "point within rounding of the upper domain face");
-    if (flag & kErrWaitTimeout) return fail(MPMGPU_ERR_DEVICE, "a bulk copy did not complete within the wait limit");
-    if (flag & kErrItemCap) return fail(MPMGPU_ERR_DEVICE, "a work item holds more points than the kernel takes");
-    return MPMGPU_OK;
+    return flag_status(flag);
   }
 
   mpmgpu_status remove_job(int job) override {
@@ -884,6 +883,135 @@ class Batch : public BatchBase {
     return MPMGPU_OK;
   }
 
+  static int field_width(int field) {
+    switch (field) {
+      case MPMGPU_P_L: case MPMGPU_P_T: return 9;
+      case MPMGPU_P_X: case MPMGPU_P_U: case MPMGPU_P_X_T: case MPMGPU_P_MX_T: return 3;
+    }
+    return 1;
+  }
+  static int host_threads() {
+    return (int)std::min<unsigned>(8, std::max(1u, std::thread::hardware_concurrency()));
+  }
+
+  // One field of several bodies converted to the reference layout on the
+  // device (k_points_field), in groups of at most kFetchGroupBytes (or one
+  // body), and delivered to the host arrays. *done = false: nothing was
+  // done, because there is no memory for the converted copy or the stream is
+  // being captured; the caller then converts on the host.
+  mpmgpu_status download_converted(const std::vector<std::pair<HBody*, double*>>& bodies, int field, int threads,
+                                   bool* done) {
+    *done = false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream_, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return MPMGPU_OK;
+    const int64_t w = field_width(field);
+    int64_t group = 1;
+    for (size_t b = 0; b < bodies.size();) {
+      int64_t sum = bodies[b].first->n * w;
+      for (b++; b < bodies.size() && (sum + bodies[b].first->n * w) * 8 <= (int64_t)kFetchGroupBytes; b++)
+        sum += bodies[b].first->n * w;
+      group = std::max(group, sum);
+    }
+    double* dev = nullptr;
+    if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&dev), (size_t)group * sizeof(double), pool_, stream_) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      return MPMGPU_OK;
+    }
+    mpmgpu_status st = MPMGPU_OK;
+    for (size_t b = 0; b < bodies.size() && st == MPMGPU_OK;) {
+      std::vector<std::pair<double*, int64_t>> segs;
+      int64_t used = 0;
+      do {
+        const HBody& B = *bodies[b].first;
+        if (B.n > 0) {
+          k_points_field<PT><<<(int)std::min<int64_t>((B.n + 255) / 256, sm_count_ * 8), 256, 0, stream_>>>(
+              B.P, dim_, field, dev + used);
+          st = check_launch("k_points_field");
+        }
+        segs.emplace_back(bodies[b].second, B.n * w);
+        used += B.n * w;
+        b++;
+      } while (b < bodies.size() && used + bodies[b].first->n * w <= group && st == MPMGPU_OK);
+      if (st == MPMGPU_OK) st = deliver(dev, used, segs, threads);
+    }
+    cudaFreeAsync(dev, stream_);
+    *done = true;
+    return st;
+  }
+
+  // Copies `total` doubles of device memory to consecutive host segments:
+  // through two pinned buffers, the next chunk under way while up to
+  // `threads` host threads copy the last one out (writing freshly mapped
+  // pages is what takes the time).
+  static constexpr int64_t kDeliverChunk = (int64_t)1 << 20;   // doubles
+  mpmgpu_status deliver(const double* dev, int64_t total, const std::vector<std::pair<double*, int64_t>>& segs,
+                        int threads) {
+    const int64_t chunk = std::min(std::max<int64_t>(total, 1), kDeliverChunk);
+    MPM_TRY(download_reserve(256 + 2 * (size_t)chunk * sizeof(double)));
+    unsigned char* base = static_cast<unsigned char*>(dl_stage_);
+    double* buf[2] = {reinterpret_cast<double*>(base + 256), reinterpret_cast<double*>(base + 256) + chunk};
+    MPM_CUDA_TRY(cudaMemcpyAsync(base, err_, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+    const int64_t chunks = (total + chunk - 1) / chunk;
+    auto queue = [&](int64_t c) {
+      const int64_t n = std::min(chunk, total - c * chunk);
+      cudaError_t e =
+          cudaMemcpyAsync(buf[c & 1], dev + c * chunk, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, stream_);
+      return e != cudaSuccess ? e : cudaEventRecord(dl_ev_[c & 1], stream_);
+    };
+    if (chunks == 0) MPM_CUDA_TRY(cudaEventRecord(dl_ev_[0], stream_));
+    if (chunks > 0) MPM_CUDA_TRY(queue(0));
+    MPM_CUDA_TRY(cudaEventSynchronize(dl_ev_[0]));
+    int flag = 0;
+    std::memcpy(&flag, base, sizeof(int));
+    MPM_TRY(flag_status(flag));
+    // values [a, b) of the whole, from chunk c's buffer
+    auto copy_out = [&](int64_t c, int64_t a, int64_t b) {
+      int64_t s0 = 0;
+      for (const auto& sg : segs) {
+        const int64_t lo = std::max(a, s0), hi = std::min(b, s0 + sg.second);
+        if (lo < hi)
+          std::memcpy(sg.first + (lo - s0), buf[c & 1] + (lo - c * chunk), (size_t)(hi - lo) * sizeof(double));
+        s0 += sg.second;
+        if (s0 >= b) break;
+      }
+    };
+    auto slice = [&](int64_t c, int t, int nt) {
+      const int64_t a = c * chunk, n = std::min(chunk, total - a);
+      copy_out(c, a + n * t / nt, a + n * (t + 1) / nt);
+    };
+    const int nt = total >= ((int64_t)1 << 18) ? std::max(1, threads) : 1;
+    // ready: chunks that have arrived; finished: slices copied out
+    std::atomic<int64_t> ready{0}, finished{0};
+    std::vector<std::thread> pool;
+    for (int t = 1; t < nt; t++)
+      pool.emplace_back([&, t]() {
+        for (int64_t c = 0; c < chunks; c++) {
+          int64_t r;
+          while ((r = ready.load(std::memory_order_acquire)) <= c && r >= 0) std::this_thread::yield();
+          if (r < 0) return;   // the copies failed
+          slice(c, t, nt);
+          finished.fetch_add(1, std::memory_order_release);
+        }
+      });
+    cudaError_t e = cudaSuccess;
+    for (int64_t c = 0; c < chunks; c++) {
+      if (c > 0) e = cudaEventSynchronize(dl_ev_[c & 1]);
+      // the other buffer was copied out in the last round
+      if (e == cudaSuccess && c + 1 < chunks) e = queue(c + 1);
+      if (e != cudaSuccess) {
+        ready.store(-1, std::memory_order_release);
+        break;
+      }
+      ready.store(c + 1, std::memory_order_release);
+      slice(c, 0, nt);
+      while (finished.load(std::memory_order_acquire) < (c + 1) * (nt - 1)) std::this_thread::yield();
+    }
+    for (auto& th : pool) th.join();
+    MPM_CUDA_TRY(e);
+    return MPMGPU_OK;
+  }
+
   mpmgpu_status download_points(int job, int body, int field, double* out) override {
     HJob* j;
     HBody* B;
@@ -896,6 +1024,9 @@ class Batch : public BatchBase {
       return MPMGPU_OK;
     }
     MPM_TRY(point_field_check(*B, field));
+    bool done = false;
+    MPM_TRY(download_converted({{B, out}}, field, host_threads(), &done));
+    if (done) return MPMGPU_OK;
     // the point ids and the arrays of the field, copied with one wait
     PointView pv;
     pv.n = n;
@@ -919,6 +1050,17 @@ class Batch : public BatchBase {
       for (int k = 0; k < count; k++) MPM_TRY(download_points(jobs[k], body, field, outs[k]));
       return MPMGPU_OK;
     }
+    std::vector<std::pair<HBody*, double*>> bodies;
+    for (int k = 0; k < count; k++) {
+      HJob* j;
+      HBody* B;
+      MPM_TRY(readable_body(jobs[k], body, &j, &B));
+      MPM_TRY(point_field_check(*B, field));
+      bodies.emplace_back(B, outs[k]);
+    }
+    bool done = false;
+    MPM_TRY(download_converted(bodies, field, std::max(1, threads), &done));
+    if (done) return MPMGPU_OK;
     std::vector<PointView> views((size_t)count);
     std::vector<std::pair<const void*, size_t>> items;
     std::vector<std::pair<size_t, const void**>> slots;   // (view, slot)
@@ -1564,24 +1706,39 @@ class Batch : public BatchBase {
     return MPMGPU_OK;
   }
 
+  // The status of the device error flags.
+  mpmgpu_status flag_status(int flag) {
+    if (flag & kErrWideSpan) return fail(MPMGPU_ERR_DEVICE, "point corners span more than two cells (extent > cell size)");
+    if (flag & kErrElemAlias) return fail(MPMGPU_ERR_DEVICE, "point within rounding of the upper domain face");
+    if (flag & kErrWaitTimeout) return fail(MPMGPU_ERR_DEVICE, "a bulk copy did not complete within the wait limit");
+    if (flag & kErrItemCap) return fail(MPMGPU_ERR_DEVICE, "a work item holds more points than the kernel takes");
+    return MPMGPU_OK;
+  }
+
+  // The pinned staging buffer of downloads, at least `bytes`.
+  mpmgpu_status download_reserve(size_t bytes) {
+    for (auto& ev : dl_ev_)
+      if (!ev) MPM_CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    if (bytes <= dl_cap_) return MPMGPU_OK;
+    MPM_CUDA_TRY(cudaStreamSynchronize(stream_));
+    pinned_give(dl_stage_, dl_cap_);
+    dl_stage_ = nullptr;
+    dl_cap_ = 0;
+    size_t cap = 0;
+    MPM_CUDA_TRY(pinned_take(bytes, &dl_stage_, &cap));
+    dl_cap_ = cap;
+    return MPMGPU_OK;
+  }
+
   // Copies device arrays to pinned staging on the compute stream (after the
   // queued work) and waits once; checks the kernels' error flag like
   // synchronize(). h[k] points at item k's bytes until the next fetch.
   mpmgpu_status fetch(const std::vector<std::pair<const void*, size_t>>& items, std::vector<const unsigned char*>& h) {
     size_t total = 256;   // error flag first
     for (auto& it : items) total += (it.second + 255) / 256 * 256;
-    if (total > dl_cap_) {
-      MPM_CUDA_TRY(cudaStreamSynchronize(stream_));
-      pinned_give(dl_stage_, dl_cap_);
-      dl_stage_ = nullptr;
-      // twice the request: the next, larger download of the same jobs (the
-      // stress after the positions) then fits without pinning pages again
-      const size_t want = std::max<size_t>(2 * total, (size_t)16 << 20);
-      dl_cap_ = 0;
-      size_t cap = 0;
-      MPM_CUDA_TRY(pinned_take(want, &dl_stage_, &cap));
-      dl_cap_ = cap;
-    }
+    // twice the request: the next, larger download of the same jobs (the
+    // stress after the positions) then fits without pinning pages again
+    if (total > dl_cap_) MPM_TRY(download_reserve(std::max<size_t>(2 * total, (size_t)16 << 20)));
     unsigned char* base = static_cast<unsigned char*>(dl_stage_);
     MPM_CUDA_TRY(cudaMemcpyAsync(base, err_, sizeof(int), cudaMemcpyDeviceToHost, stream_));
     size_t off = 256;
@@ -1594,11 +1751,7 @@ class Batch : public BatchBase {
     MPM_CUDA_TRY(cudaStreamSynchronize(stream_));
     int flag = 0;
     std::memcpy(&flag, base, sizeof(int));
-    if (flag & kErrWideSpan) return fail(MPMGPU_ERR_DEVICE, "point corners span more than two cells (extent > cell size)");
-    if (flag & kErrElemAlias) return fail(MPMGPU_ERR_DEVICE, "point within rounding of the upper domain face");
-    if (flag & kErrWaitTimeout) return fail(MPMGPU_ERR_DEVICE, "a bulk copy did not complete within the wait limit");
-    if (flag & kErrItemCap) return fail(MPMGPU_ERR_DEVICE, "a work item holds more points than the kernel takes");
-    return MPMGPU_OK;
+    return flag_status(flag);
   }
 
   template <typename T>
@@ -2446,11 +2599,7 @@ class Batch : public BatchBase {
     frame_.pending = false;
     MPM_CUDA_TRY(cudaEventSynchronize(frame_ev_));
     const int flag = *frame_.err;
-    if (flag & kErrWideSpan) return fail(MPMGPU_ERR_DEVICE, "point corners span more than two cells (extent > cell size)");
-    if (flag & kErrElemAlias) return fail(MPMGPU_ERR_DEVICE, "point within rounding of the upper domain face");
-    if (flag & kErrWaitTimeout) return fail(MPMGPU_ERR_DEVICE, "a bulk copy did not complete within the wait limit");
-    if (flag & kErrItemCap) return fail(MPMGPU_ERR_DEVICE, "a work item holds more points than the kernel takes");
-    return MPMGPU_OK;
+    return flag_status(flag);
   }
 
   mpmgpu_status frame_body(int job, int body, HBody** B) {
@@ -2512,6 +2661,7 @@ class Batch : public BatchBase {
   int32_t* cell_count_ = nullptr;
   int64_t cap_cells_ = 0;
   void* dl_stage_ = nullptr;   // pinned staging of downloads
+  cudaEvent_t dl_ev_[2] = {nullptr, nullptr};   // its two halves' copies (deliver)
   size_t dl_cap_ = 0;
   unsigned long long* cell_hist_ = nullptr;   // per cell: 8 class counts of 8 bits
   int64_t cap_cells_h_ = 0;
