@@ -410,6 +410,7 @@ class Batch : public BatchBase {
     if (det_ && mixed()) return fail(MPMGPU_ERR_UNSUPPORTED, "the deterministic form is FP64");
     MPM_TRY(alloc_raw(&hdr_, 1, scratch_allocs_));
     MPM_TRY(alloc_raw(&count_, 1, scratch_allocs_));
+    MPM_TRY(alloc_raw(&active_acc_, 1, scratch_allocs_));
     MPM_TRY(alloc_raw(&err_, 1, scratch_allocs_));
     MPM_TRY(alloc_raw(&drift_, 1, scratch_allocs_));
     MPM_TRY(alloc_raw(&queue_, 2, scratch_allocs_));
@@ -2138,6 +2139,12 @@ class Batch : public BatchBase {
   template <int DIM, int CAP, bool NORMAL, bool SINGLE, bool DET>
   mpmgpu_status launch_fused_k(int prime_pass, int phases, int one_body, cudaStream_t st) {
     FusedLaunch<PT> fl{};
+    if (publish_ && !prime_pass) {
+      fl.active_acc = active_acc_;
+      fl.active_pub = active_nodes_;
+      fl.blocks = count_;
+      publish_ = false;
+    }
     if (SINGLE) fl.one = ctx_host_[(size_t)one_body];
     fl.one_body = SINGLE ? one_body : -1;
     fl.bodies = ctx_d_;
@@ -2195,6 +2202,12 @@ class Batch : public BatchBase {
   template <int NT, int PPT, bool NORMAL, bool SINGLE, int MAT>
   mpmgpu_status launch_lean_k(int prime_pass, int phases, int one_body, cudaStream_t st) {
     FusedLaunch<PT> fl{};
+    if (publish_ && !prime_pass) {
+      fl.active_acc = active_acc_;
+      fl.active_pub = active_nodes_;
+      fl.blocks = count_;
+      publish_ = false;
+    }
     if (SINGLE) fl.one = ctx_host_[(size_t)one_body];
     fl.one_body = SINGLE ? one_body : -1;
     fl.bodies = ctx_d_;
@@ -2335,21 +2348,32 @@ class Batch : public BatchBase {
   }
 
   mpmgpu_status launch_step_direct() {
-    {
-      StageTimer timer(this, kStageCompact);
-      MPM_CUDA_TRY(cudaMemsetAsync(count_, 0, sizeof(unsigned long long), stream_));
-      k_compact<<<stride_blocks(256), 256, 0, stream_>>>(hdr_, flags_, list_, count_, was_active_, active_nodes_);
-      MPM_TRY(check_launch("k_compact"));
-    }
-    {
+    if (hdr_host_.blocks <= kScanBlocks) {
+      StageTimer timer(this, kStageGrid);
+      const int gb = (int)std::max<int64_t>(1, std::min<int64_t>(sm_count_ * 8, (hdr_host_.blocks + 3) / 4));
+      if (dim_ == 3)
+        k_grid_scan<3><<<gb, kGridThreads, 0, stream_>>>(hdr_, insts_d_, gbodies_d_, blk_inst_, flags_, was_active_,
+                                                         active_acc_);
+      else
+        k_grid_scan<2><<<gb, kGridThreads, 0, stream_>>>(hdr_, insts_d_, gbodies_d_, blk_inst_, flags_, was_active_,
+                                                         active_acc_);
+      MPM_TRY(check_launch("k_grid_scan"));
+    } else {
+      {
+        StageTimer timer(this, kStageCompact);
+        const int64_t cb = std::min<int64_t>(stride_blocks(256), (hdr_host_.blocks + 255) / 256);
+        k_compact<<<(int)cb, 256, 0, stream_>>>(hdr_, flags_, list_, count_, was_active_);
+        MPM_TRY(check_launch("k_compact"));
+      }
       StageTimer timer(this, kStageGrid);
       const int gb = sm_count_ * 32;
       if (dim_ == 3)
-        k_grid<3><<<gb, 64, 0, stream_>>>(insts_d_, gbodies_d_, blk_inst_, list_, count_, active_nodes_);
+        k_grid<3><<<gb, 64, 0, stream_>>>(insts_d_, gbodies_d_, blk_inst_, list_, count_, active_acc_);
       else
-        k_grid<2><<<gb, 64, 0, stream_>>>(insts_d_, gbodies_d_, blk_inst_, list_, count_, active_nodes_);
+        k_grid<2><<<gb, 64, 0, stream_>>>(insts_d_, gbodies_d_, blk_inst_, list_, count_, active_acc_);
       MPM_TRY(check_launch("k_grid"));
     }
+    publish_ = true;   // the step's first fused launch closes the grid update's counts
     if (det_) {
       // update, bounds from the new state, then the scatter
       MPM_TRY(launch_fused(0, 1));
@@ -2633,7 +2657,11 @@ class Batch : public BatchBase {
   // device tables and scratch
   BatchHdr* hdr_ = nullptr;
   BatchHdr hdr_host_{};
+  // blocks listed and nodes with mass counted by the grid update under way,
+  // both zero between steps (publish_counts)
   unsigned long long* count_ = nullptr;
+  unsigned long long* active_acc_ = nullptr;
+  bool publish_ = false;
   int* err_ = nullptr;
   unsigned long long* drift_ = nullptr;
   int* queue_ = nullptr;   // the fused kernels' work queue (claim_item), zero between launches

@@ -68,6 +68,12 @@ struct FusedLaunch {
   // out flags kErrWaitTimeout and its CTA returns (after the copies in
   // flight have landed, waited for with the default limit)
   uint32_t wait_polls;
+  // the grid update's counts, closed by the step's first launch after it (null
+  // in the others): the nodes with mass are published, *active_pub =
+  // *active_acc, and that count and the listed blocks start from zero again
+  unsigned long long* active_acc;
+  unsigned long long* active_pub;
+  unsigned long long* blocks;
   // work queue of the launch (two counters, zero between launches; see
   // claim_item)
   int* queue;
@@ -96,6 +102,15 @@ __device__ __forceinline__ void queue_done(int* queue) {
   if (atomicAdd(queue + 1, 1) == (int)gridDim.x - 1) {
     atomicExch(queue, 0);
     atomicExch(queue + 1, 0);
+  }
+}
+
+template <typename PT>
+__device__ __forceinline__ void publish_counts(const FusedLaunch<PT>& fl) {
+  if (fl.active_acc != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
+    *fl.active_pub = *fl.active_acc;
+    *fl.active_acc = 0;
+    *fl.blocks = 0;
   }
 }
 
@@ -893,6 +908,7 @@ __global__ void __launch_bounds__(fused_threads<PT, CAP>(), fused_min_ctas<PT, C
   // after the accumulator levels (two in the deterministic form)
   uint8_t* touched = smem + off_touched<DIM, PT, CAP, NORMAL, DET>();
 
+  publish_counts(fl);
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
     mbar_init(bar_ctx, 1);

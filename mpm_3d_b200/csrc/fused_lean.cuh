@@ -771,6 +771,7 @@ __global__ void __launch_bounds__(NT, lean_min_ctas<PT, NT, PPT>())
   sh.far = reinterpret_cast<uint16_t*>(smem + lean_off_far<DIM, PT, CAP>());
   sh.cells = smem + lean_off_far<DIM, PT, CAP>() + sizeof(uint16_t) * CAP;
 
+  publish_counts(fl);
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
     mbar_init(bar_ctx, 1);
