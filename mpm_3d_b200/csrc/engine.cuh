@@ -175,7 +175,7 @@ inline int64_t job_footprint(const mpmgpu_config& cfg, int mode, bool keep_debug
     if (keep_debug && !mixed) bytes += 2 * n * 72;
     bytes += g.nslots * 8 * (7 + 6);            // accumulators + velocities
     if (mode == MPMGPU_MODE_FP64_DETERMINISTIC) bytes += g.nslots * 8 * 7;
-    bytes += n * 10;                             // sort key, rank, class rank
+    bytes += n * 14;                             // sort key, rank, class rank, source
     bytes += ((int64_t)bg.nbins * bg.cells_per_bin + 1) * 12 + ((int64_t)bg.nbins + 2) * 4;
     bytes += ((int64_t)bg.nbins + n / 256 + 1) * 16;
     if (keep_debug) bytes += g.nslots * 8 * 7;
@@ -2017,6 +2017,7 @@ class Batch : public BatchBase {
     MPM_TRY(grow(&list_, &tmp_cap, cap_blocks_, 0));
     MPM_TRY(grow(&key_, &cap_points_k_, std::max<int64_t>(points, 1), 0));
     MPM_TRY(grow(&rank_, &cap_points_r_, std::max<int64_t>(points, 1), 0));
+    MPM_TRY(grow(&src_, &cap_points_s_, std::max<int64_t>(points, 1), 0));
     MPM_TRY(grow(&cell_count_, &cap_cells_, std::max<int64_t>(cells, 1), 0));
     MPM_TRY(grow(&cell_hist_, &cap_cells_h_, std::max<int64_t>(cells, 1), 0));
     MPM_TRY(grow(&crank_, &cap_points_c_, std::max<int64_t>(points, 1), 0));
@@ -2400,10 +2401,12 @@ class Batch : public BatchBase {
     MPM_TRY(check_launch("k_scan_small"));
     k_scan_add<<<chunks, kScanChunk, 0, stream_>>>(hdr_, bin_scan_, chunk_sum_);
     MPM_TRY(check_launch("k_scan_add"));
-    k_sort_scatter<DIM, PT><<<sb, 256, 0, stream_>>>(hdr_, ctx_d_, point_end_d_, key_, rank_, cell_count_, cell_hist_,
-                                                     crank_, bin_scan_);
-    MPM_TRY(check_launch("k_sort_scatter"));
-    k_sort_flip<PT><<<std::max(1, (hdr_host_.nbodies + 255) / 256 + 1), 256, 0, stream_>>>(hdr_, ctx_d_);
+    k_sort_place<DIM, PT><<<sb, 256, 0, stream_>>>(hdr_, ctx_d_, point_end_d_, key_, rank_, cell_count_, cell_hist_,
+                                                   crank_, bin_scan_, src_);
+    MPM_TRY(check_launch("k_sort_place"));
+    k_sort_gather<DIM, PT><<<sb, 256, 0, stream_>>>(hdr_, ctx_d_, point_end_d_, src_);
+    MPM_TRY(check_launch("k_sort_gather"));
+    k_sort_flip<PT><<<std::max(1, std::min(hdr_host_.nbodies, sm_count_ * 8)), 64, 0, stream_>>>(hdr_, ctx_d_);
     MPM_TRY(check_launch("k_sort_flip"));
     k_bin_work<PT><<<sb, 256, 0, stream_>>>(hdr_, ctx_d_, bin_end_d_, bin_scan_, item_off_d_, cap_, work_bin_,
                                             work_start_, work_end_, nwork_body_);
@@ -2686,6 +2689,8 @@ class Batch : public BatchBase {
   int64_t cap_points_k_ = 0;
   int32_t* rank_ = nullptr;
   int64_t cap_points_r_ = 0;
+  int32_t* src_ = nullptr;     // per destination of a re-binning: the point that goes there
+  int64_t cap_points_s_ = 0;
   int32_t* cell_count_ = nullptr;
   int64_t cap_cells_ = 0;
   void* dl_stage_ = nullptr;   // pinned staging of downloads

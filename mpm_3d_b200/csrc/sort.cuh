@@ -27,6 +27,8 @@
 // their bin's tile.
 #pragma once
 
+#include <cstddef>
+
 #include "geom.cuh"
 #include "state.cuh"
 
@@ -157,25 +159,33 @@ __global__ void k_sort_count(const BatchHdr* hdr, const BodyCtx<PT>* bodies, con
   }
 }
 
-// Pass 2: per-bin point counts (one thread per bin entry, summing its
-// cells); entry nbins of a body counts its inactive points.
+// Pass 2: per-bin point counts; entry nbins of a body counts its inactive
+// points. Sixteen lanes per bin entry, four cells each: a bin's 64 counters
+// are one 256-byte read (21 block drops, 2.6 M points: one thread per bin,
+// counter after counter, 46 us; 16 lanes 19 us).
 template <typename PT>
 __global__ void k_bin_totals(const BatchHdr* hdr, const BodyCtx<PT>* bodies, const int64_t* bin_end,
                              const int32_t* cell_count, int32_t* bin_total) {
   const int64_t total = hdr->bins;
   const int nb = hdr->nbodies;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += stride) {
-    const BodyCtx<PT>& B = bodies[find_range(bin_end, nb, i)];
-    const int lb = (int)(i - B.bin_off);
-    const int32_t* cc = cell_count + B.cell_off;
+  const int lane = threadIdx.x & 15;
+  const int64_t stride = ((int64_t)gridDim.x * blockDim.x) >> 4;
+  for (int64_t i0 = (blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31)) >> 4; i0 < total; i0 += stride) {
+    const int64_t i = i0 + ((threadIdx.x >> 4) & 1);   // whole warps stay in the loop for the shuffles
     int s = 0;
-    if (lb < B.bg.nbins) {
-      for (int l = 0; l < B.bg.cells_per_bin; l++) s += cc[lb * B.bg.cells_per_bin + l];
-    } else {
-      s = cc[B.bg.nbins * B.bg.cells_per_bin];
+    if (i < total) {
+      const BodyCtx<PT>& B = bodies[find_range(bin_end, nb, i)];
+      const int lb = (int)(i - B.bin_off);
+      const int32_t* cc = cell_count + B.cell_off + (int64_t)lb * B.bg.cells_per_bin;
+      if (lb < B.bg.nbins) {
+        for (int l = lane; l < B.bg.cells_per_bin; l += 16) s += cc[l];
+      } else if (lane == 0) {
+        s = cc[0];
+      }
     }
-    bin_total[i] = s;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0 && i < total) bin_total[i] = s;
   }
 }
 
@@ -265,8 +275,8 @@ __global__ void __launch_bounds__(kScanChunk) k_scan_add(const BatchHdr* hdr, in
   if (i < n) v[i] += chunk_sum[blockIdx.x];
 }
 
-// Pass 3: destination of each point inside its bin (rank-major order) and
-// the permutation copy of every per-point array into the second buffer.
+// Pass 3: destination of each point inside its bin (rank-major order); the
+// point's index goes to `src` there.
 // The rank of a point within its cell is its class-order rank (points of
 // lower classes first, then the class's arrival rank) when the cell's class
 // histogram is exact, i.e. its counts sum to the cell's count (a class of
@@ -274,9 +284,10 @@ __global__ void __launch_bounds__(kScanChunk) k_scan_add(const BatchHdr* hdr, in
 // otherwise every point of that cell keeps its arrival rank. Either way the
 // ranks of a cell are a permutation of 0 .. count-1.
 template <int DIM, typename PT>
-__global__ void k_sort_scatter(const BatchHdr* hdr, const BodyCtx<PT>* bodies, const int64_t* point_end,
-                               const int32_t* key, const int32_t* rank, const int32_t* cell_count,
-                               const unsigned long long* cell_hist, const int16_t* crank, const int32_t* bin_scan) {
+__global__ void k_sort_place(const BatchHdr* hdr, const BodyCtx<PT>* bodies, const int64_t* point_end,
+                             const int32_t* key, const int32_t* rank, const int32_t* cell_count,
+                             const unsigned long long* cell_hist, const int16_t* crank, const int32_t* bin_scan,
+                             int32_t* src) {
   const int64_t total = hdr->points;
   const int nb = hdr->nbodies;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -313,45 +324,84 @@ __global__ void k_sort_scatter(const BatchHdr* hdr, const BodyCtx<PT>* bodies, c
     } else {
       pos += r;
     }
+    src[B.point_off + pos] = (int32_t)p;
+  }
+}
+
+// Pass 4: the permutation copy of every per-point array into the second
+// buffer, one thread per destination: the writes are whole lines, and the
+// scattered 8-byte reads of a bin's points, which lie together since the last
+// re-binning, meet in L1 (2.6 M points from their input order: one thread per
+// source with scattered writes 850 us, placing included; 124 us to place and
+// 252 us to copy now, 778 MB in and out at 3.1 TB/s). A thread has all the
+// loads of a group of arrays in flight before its first store.
+template <int DIM, typename PT>
+__global__ void __launch_bounds__(256) k_sort_gather(const BatchHdr* hdr, const BodyCtx<PT>* bodies,
+                                                     const int64_t* point_end, const int32_t* src) {
+  const int64_t total = hdr->points;
+  const int nb = hdr->nbodies;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += stride) {
+    const BodyCtx<PT>& B = bodies[find_range(point_end, nb, q)];
+    const int64_t pos = q - B.point_off;
+    const int64_t p = src[q];
     const PointsT<PT>& S = B.P;
     const PointsT<PT>& D = B.Palt;
+    // the arrays x v u s vol m ext follow one another in PointsT
+    const PT* const* sa = &S.x[0];
+    PT* const* da = &D.x[0];
+    constexpr int kArrays = 18, kGroup = 9;
+    static_assert(offsetof(PointsT<PT>, ext) == offsetof(PointsT<PT>, x) + (kArrays - 1) * sizeof(PT*),
+                  "the copied arrays are consecutive members");
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-      D.x[d][pos] = S.x[d][p];
-      D.v[d][pos] = S.v[d][p];
-      D.u[d][pos] = S.u[d][p];
+    for (int g = 0; g < kArrays; g += kGroup) {
+      PT v[kGroup];
+#pragma unroll
+      for (int f = 0; f < kGroup; f++) v[f] = sa[g + f][p];
+#pragma unroll
+      for (int f = 0; f < kGroup; f++) da[g + f][pos] = v[f];
     }
-#pragma unroll
-    for (int c = 0; c < 6; c++) D.s[c][pos] = S.s[c][p];
-    D.vol[pos] = S.vol[p];
-    D.m[pos] = S.m[p];
-    D.ext[pos] = S.ext[p];
-    D.active[pos] = S.active[p];
-    D.pid[pos] = S.pid[p];
+    const int32_t act = S.active[p], id = S.pid[p];
+    D.active[pos] = act;
+    D.pid[pos] = id;
     if (S.L != nullptr)
       for (int a = 0; a < 9; a++) D.L[9 * pos + a] = S.L[9 * p + a];
 #pragma unroll
     for (int a = 0; a < 9; a++)
       if (S.ms[a] != nullptr) D.ms[a][pos] = S.ms[a][p];
     if (S.ml != nullptr) {
+      PT v[7];
 #pragma unroll
       for (int d = 0; d < 3; d++) {
-        D.xl[d][pos] = S.xl[d][p];
-        D.vl[d][pos] = S.vl[d][p];
+        v[d] = S.xl[d][p];
+        v[3 + d] = S.vl[d][p];
       }
-      D.ml[pos] = S.ml[p];
+      v[6] = S.ml[p];
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        D.xl[d][pos] = v[d];
+        D.vl[d][pos] = v[3 + d];
+      }
+      D.ml[pos] = v[6];
     }
   }
 }
 
-// Swaps the two point buffers of every body after the scatter.
+// Swaps the two point buffers of every body after the copy: one CTA of 64
+// threads per body, one 8-byte word each (one thread per body, with the
+// structures through local memory, took 14 us).
 template <typename PT>
-__global__ void k_sort_flip(const BatchHdr* hdr, BodyCtx<PT>* bodies) {
+__global__ void __launch_bounds__(64) k_sort_flip(const BatchHdr* hdr, BodyCtx<PT>* bodies) {
+  static_assert(sizeof(PointsT<PT>) % 8 == 0 && sizeof(PointsT<PT>) / 8 <= 64, "one word per thread");
   const int nb = hdr->nbodies;
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-    const PointsT<PT> t = bodies[b].P;
-    bodies[b].P = bodies[b].Palt;
-    bodies[b].Palt = t;
+  const int w = threadIdx.x;
+  for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+    if (w >= (int)(sizeof(PointsT<PT>) / 8)) continue;
+    uint64_t* cur = reinterpret_cast<uint64_t*>(&bodies[b].P) + w;
+    uint64_t* alt = reinterpret_cast<uint64_t*>(&bodies[b].Palt) + w;
+    const uint64_t t = *cur;
+    *cur = *alt;
+    *alt = t;
   }
 }
 
