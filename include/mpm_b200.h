@@ -77,7 +77,8 @@ typedef struct {
   int keep_debug;   /* 1: keep L, nodal m/mx_t/f and contact forces
                        readable after each step (costs extra traffic) */
   int sort_interval;/* steps between re-binning the points by cell
-                       (0 = default 32); results do not depend on it */
+                       (0 = default: 32, or 16 with more than four bodies);
+                       results do not depend on it */
 } mpmgpu_config;
 
 /* One DefaultBody: its points (DefaultPoints::readFromFile columns,
@@ -286,16 +287,16 @@ typedef enum {
    * 1024 (3D mixed), 512 (2D); the only form of 2D jobs and of the
    * deterministic form */
   MPMGPU_KERNEL_STAGED = 0,
-  /* each thread takes its points from gather to scatter, point state read
-   * from global memory: 128 points per item (CTAs of 128 threads), 256
-   * (256 threads) or 512 (256 threads, two points each); 3D, not the
-   * deterministic form */
+  /* each thread takes its points from gather to their new map, then four
+   * threads per cell sum the cell's points: 128 points per item (CTAs of 128
+   * threads), 256 (256 threads) or 512 (256 threads, two points each); 3D,
+   * not the deterministic form */
   MPMGPU_KERNEL_POINT_PER_THREAD = 1
 } mpmgpu_kernel_form;
 
 /* Selects the fused kernel's form and points per work item (default: one
- * point per thread with 512 points in 3D outside the deterministic form,
- * else staged with 512); MPMGPU_ERR_ARG if the pair is not available for
+ * point per thread in 3D outside the deterministic form, with 512 points, or
+ * 128 for jobs of up to 65,536 points in all, else staged with 512); MPMGPU_ERR_ARG if the pair is not available for
  * the handle. Takes effect at the next step. */
 mpmgpu_status mpmgpu_set_kernel(mpmgpu_handle* h, int form, int points_per_item);
 mpmgpu_status mpmgpu_kernel(const mpmgpu_handle* h, int* form, int* points_per_item);
@@ -342,10 +343,12 @@ typedef struct {
   int dim;             /* 2 or 3 for every job of the batch */
   int mode;            /* MPMGPU_MODE_FP64 or MPMGPU_MODE_MIXED */
   int device;          /* CUDA device ordinal */
-  int sort_interval;   /* steps between re-binnings (0 = default 32) */
+  int sort_interval;   /* steps between re-binnings (0 = default: 32 with up
+                          to four bodies in the batch, 16 with more) */
   int points_per_item; /* points per CTA work item: 0 = default (3D,
                           not deterministic: 512 on the point-per-thread
-                          kernel; else 512 on the staged kernel); 128, 256
+                          kernel, 128 while the jobs have up to 65,536
+                          points in all; else 512 on the staged kernel); 128, 256
                           or 512 run on the point-per-thread kernel where
                           it applies, other sizes on the staged kernel
                           (1024 in the 3D mixed form, 512 in 2D); see

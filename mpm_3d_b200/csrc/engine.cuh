@@ -141,6 +141,24 @@ inline bool cap_available(int dim, bool mixed, int cap) {
   return cap == 512;
 }
 
+// Points of the stepped jobs up to which the point-per-thread kernel takes
+// items of 128 points by default: such jobs are a few items per SM or less,
+// and the time of a step is that of one item. Measured (us per step, 512 ->
+// 128): 1,728 points 27.8 -> 23.1, 43,904 sand points 28.4 -> 24.1, two
+// bodies of 27,000 points 35.6 -> 32.9, of 32,768 points 37.6 -> 36.5; column
+// of 96,000 points 28.5 -> 32.7, 128,000 sand points 32.8 -> 40.6.
+constexpr int64_t kSmallPoints = 65536;
+
+// Default steps between re-binnings: 32 for up to four bodies, 16 for more
+// (launches over the body table), whose jobs move at unlike speeds and are
+// re-binned together. A point that has drifted out of its item's tile takes
+// a general path through global memory, and its warp waits: of 21 block drops
+// in 2.6 M points 3.4 % of the visits at an interval of 32, 0.4 % at 16 (727
+// -> 681 us per step; 692 at 20, 668 at 12, 678 at 8; mixed, 0.5 M points:
+// 179 -> 173, 176 at 12). Bodies that hardly drift pay for the re-binning
+// alone: column 384 us at 32, 395 at 16.
+constexpr int kSortInterval = 32, kSortIntervalTable = 16;
+
 // Forms of the fused kernel (mpmgpu_set_kernel): the staged kernel
 // (fused.cuh: point arrays staged in shared memory, gather and scatter
 // phases apart, up to 1024 points per CTA) and the point-per-thread kernel
@@ -382,7 +400,8 @@ class Batch : public BatchBase {
 
   Batch(int dim, int device, int sort_interval, int cap, int use_graph, int keep_debug, bool det = false)
       : dim_(dim), device_(device), keep_debug_(keep_debug != 0), use_graph_(use_graph != 0), det_(det) {
-    sort_interval_ = sort_interval > 0 ? sort_interval : 32;
+    sort_interval_ = sort_interval > 0 ? sort_interval : kSortInterval;
+    sort_auto_ = sort_interval <= 0;
     cap_ = cap;
   }
 
@@ -403,6 +422,7 @@ class Batch : public BatchBase {
     MPM_CUDA_TRY(shared_pool(device_, &pool_));
     // a requested item size is served by the point-per-thread kernel
     // where it has that size, else by the staged kernel
+    cap_auto_ = cap_ == 0;
     if (cap_ == 0) cap_ = (dim_ == 3 && !det_) ? kDefaultLeanCap : default_cap();
     form_ = form_available(dim_, mixed(), det_, kFormLean, cap_) ? kFormLean : kFormStaged;
     if (!form_available(dim_, mixed(), det_, form_, cap_) || (det_ && cap_ != default_cap()))
@@ -1443,6 +1463,7 @@ class Batch : public BatchBase {
     MPM_TRY(commit());
     if (live_jobs_ == 0) return fail(MPMGPU_ERR_STATE, "no jobs to tune on");
     MPM_TRY(snapshot_save());
+    cap_auto_ = sort_auto_ = false;   // from here on the tuner's choices
     const int original_cap = cap_, original_si = sort_interval_;
     cudaEvent_t e0, e1;
     MPM_CUDA_TRY(cudaEventCreate(&e0));
@@ -1519,6 +1540,7 @@ class Batch : public BatchBase {
     if (!form_available(dim_, mixed(), det_, form, cap) || (det_ && cap != default_cap()))
       return fail(MPMGPU_ERR_ARG, "kernel form " + std::to_string(form) + " with " + std::to_string(cap) +
                                       " points per item is not available for this batch");
+    cap_auto_ = false;
     if (form == form_ && cap == cap_) return MPMGPU_OK;
     form_ = form;
     cap_ = cap;
@@ -2035,6 +2057,10 @@ class Batch : public BatchBase {
     for (size_t b = 0; b < ctx.size(); b++) ctx[b].flags = flags_ + insts[(size_t)ctx[b].inst].block_off;
     ctx_host_ = ctx;
     single_mode_ = ctx.size() <= (size_t)kSideStreams + 1;   // one launch per body, concurrent (one_body_launches)
+    // the defaults follow the jobs (the work list is rebuilt below whenever
+    // the membership changes)
+    if (membership && cap_auto_ && form_ == kFormLean) cap_ = points <= kSmallPoints ? 128 : kDefaultLeanCap;
+    if (sort_auto_) sort_interval_ = single_mode_ ? kSortInterval : kSortIntervalTable;
     any_plain_ = any_normal_ = false;
     all_elastic_ = true;
     for (const auto& c : ctx) {
@@ -2585,6 +2611,7 @@ class Batch : public BatchBase {
   bool det_ = false;   // deterministic form: two-level exact nodal sums
   int sort_interval_ = 32;
   int cap_ = 512;
+  bool cap_auto_ = false, sort_auto_ = false;   // chosen by the defaults' rules, not by the caller
   int sm_count_ = 148;
   int fused_per_sm_[24] = {};
   cudaStream_t copy_stream_ = nullptr;
