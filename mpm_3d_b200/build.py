@@ -24,8 +24,10 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-Xcompiler", "-fPIC",
     "-shared",
-    # the optimiser takes the translation unit's kernels in parallel
-    "-split-compile", "0",
+    # the optimiser takes the translation unit's kernels in parallel, in a
+    # fixed number of parts: how the unit is cut can show in the kernels' code,
+    # so it must not follow the machine's cores
+    "-split-compile", "8",
 ]
 
 
