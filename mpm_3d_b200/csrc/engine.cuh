@@ -26,6 +26,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <memory>
 #include <set>
 #include <mutex>
@@ -1001,11 +1002,14 @@ class Batch : public BatchBase {
       const int64_t a = c * chunk, n = std::min(chunk, total - a);
       copy_out(c, a + n * t / nt, a + n * (t + 1) / nt);
     };
-    const int nt = total >= ((int64_t)1 << 18) ? std::max(1, threads) : 1;
-    // ready: chunks that have arrived; finished: slices copied out
+    // ready: chunks that have arrived; finished: slices copied out; nt: the
+    // threads there are, this one included (set before the first chunk is
+    // announced; fewer than asked for if the system has no more)
     std::atomic<int64_t> ready{0}, finished{0};
+    int nt = 1;
     std::vector<std::thread> pool;
-    for (int t = 1; t < nt; t++)
+    const int want = total >= ((int64_t)1 << 18) ? std::max(1, threads) : 1;
+    auto start = [&](int t) {
       pool.emplace_back([&, t]() {
         for (int64_t c = 0; c < chunks; c++) {
           int64_t r;
@@ -1015,6 +1019,12 @@ class Batch : public BatchBase {
           finished.fetch_add(1, std::memory_order_release);
         }
       });
+    };
+    try {
+      for (int t = 1; t < want; t++) start(t);
+    } catch (const std::exception&) {
+    }
+    nt = 1 + (int)pool.size();
     cudaError_t e = cudaSuccess;
     for (int64_t c = 0; c < chunks; c++) {
       if (c > 0) e = cudaEventSynchronize(dl_ev_[c & 1]);
