@@ -474,6 +474,38 @@ __device__ __forceinline__ void store_two(PT* sp, const PointsT<PT>& P, int64_t 
   }
 }
 
+// Adds what the reference velocity of the mixed form contributes to the sums
+// gathered from v - vref: vref itself to S^T v, since the weights sum to one
+// and every gradient's to zero, or in a map that is only partial vref times
+// those sums.
+template <int DIM, typename R>
+__device__ __forceinline__ void add_reference(const PointMapT<R>& pm, const double* vref, GatherSum<R>& gs) {
+  if (!pm.partial) {
+#pragma unroll
+    for (int d = 0; d < DIM; d++) gs.du[d] += (R)vref[d];
+    return;
+  }
+  // per axis: the weights sum to 2 (corner-sampled, both corners with an
+  // element) or 1, and the gradients of the former to zero exactly
+  const bool sampled = pm.sS == R(1);
+  R ws[3] = {R(1), R(1), R(1)}, gsum[3] = {R(0), R(0), R(0)};
+#pragma unroll
+  for (int d = 0; d < DIM; d++) {
+    const bool both = !sampled && pm.ax[d].W[0] + pm.ax[d].W[1] + pm.ax[d].W[2] > R(1.5);
+    ws[d] = both ? R(2) : R(1);
+    gsum[d] = both ? R(0) : pm.ax[d].G[0] + pm.ax[d].G[1];
+  }
+  const R S = pm.sS * (ws[0] * ws[1] * ws[2]);
+  const R g[3] = {pm.sG * gsum[0] * (ws[1] * ws[2]), pm.sG * gsum[1] * (ws[0] * ws[2]),
+                  pm.sG * gsum[2] * (ws[0] * ws[1])};
+#pragma unroll
+  for (int d = 0; d < DIM; d++) {
+    gs.du[d] += S * (R)vref[d];
+#pragma unroll
+    for (int b = 0; b < DIM; b++) gs.L[d][b] += g[b] * (R)vref[d];
+  }
+}
+
 // Phase 1 for one point: gather, movePoints / calculateStrainRate /
 // updateDensity / updateStress (explicit_usl.cpp:266-355). `sp` points at the
 // point's column in the staged arrays (stride ROW).
@@ -509,10 +541,7 @@ __device__ __forceinline__ void gather_update(const BodyCtx<PT>& c, int* err, un
       gs = gather_box_any<DIM, T, TN>(pm, o, tvel, __reduce_or_sync(inm, span_bits<DIM>(pm)));
     else
       gs = gather_general<DIM, T, TN>(c, drift, pm, o, tvel, vref);
-    if constexpr (sizeof(PT) == 4) {
-#pragma unroll
-      for (int d = 0; d < DIM; d++) gs.du[d] += (R)vref[d];
-    }
+    if constexpr (sizeof(PT) == 4) add_reference<DIM>(pm, vref, gs);
   }
   // movePoints: u_node = dt * x_t_node; x += S^T u, u += S^T u,
   // x_t += S^T diff_x_t (explicit_usl.cpp:279-292); the mixed form adds

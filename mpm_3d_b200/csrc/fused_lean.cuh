@@ -490,10 +490,7 @@ __device__ __forceinline__ void lean_far_point(const BodyCtx<PT>& c, int* err, u
     GatherSum<R> gs;
     if (build_map<3>(c.g, c.mc, c.sp.cpdi, x, ext, pm, err) > 0) {
       gs = gather_general<3, kLeanSide + 1, 1>(c, drift, pm, o, (const R*)nullptr, vref);
-      if constexpr (sizeof(PT) == 4) {
-#pragma unroll
-        for (int d = 0; d < 3; d++) gs.du[d] += (R)vref[d];
-      }
+      if constexpr (sizeof(PT) == 4) add_reference<3>(pm, vref, gs);
     }
     const R u[3] = {P.u[0][p], P.u[1][p], P.u[2][p]};
     lean_update<MAT>(c, p, gs, x, vd, u, vol, s6, MAT == 2 || MAT < 0 ? P.m[p] : R(0));

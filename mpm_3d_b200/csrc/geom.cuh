@@ -86,6 +86,9 @@ struct PointMapT {
   AxisMapT<R> ax[3];
   R sS;
   R sG;
+  // mixed form: the weights do not sum to one or a gradient's weights not to
+  // zero (an upper corner without an element; a sampled point on a node)
+  bool partial;
 };
 using AxisMap = AxisMapT<double>;
 using PointMap = PointMapT<double>;
@@ -245,6 +248,7 @@ __device__ __forceinline__ int build_map_f32(const Geom& g, const MapConst& mc, 
   int cpdi = cpdi_spec;
   const double a = 0.5 * (double)extent;
   double clo[3], chi[3];
+  pm.partial = false;
 #pragma unroll
   for (int d = 0; d < DIM; d++) {
     clo[d] = x[d] - a;
@@ -270,6 +274,7 @@ __device__ __forceinline__ int build_map_f32(const Geom& g, const MapConst& mc, 
       if (delta > 1 || delta < 0) atomicOr(err, kErrWideSpan);
       A.base = elo;
       A.span = 2 + (hi_ok && delta == 1 ? 1 : 0);
+      if (!hi_ok) pm.partial = true;
       const float rl = (float)((clo[d] - g.h[d] * (double)elo) * mc.invh[d]);
       const float wl0 = 1.0f - fabsf(rl), wl1 = 1.0f - fabsf(rl - 1.0f);
       float wh0 = 0.0f, wh1 = 0.0f;
@@ -319,6 +324,7 @@ __device__ __forceinline__ int build_map_f32(const Geom& g, const MapConst& mc, 
     }
     A.W[2] = 0.0f;
     A.G[2] = 0.0f;
+    if (A.G[0] + A.G[1] != 0.0f) pm.partial = true;
   }
   pm.sS = 1.0f;
   pm.sG = 1.0f;
