@@ -212,17 +212,24 @@ __device__ __forceinline__ int lean_element(const MapConst& mc, int d, double c,
   off = off + (below ? 1.0 : 0.0);
   return __double2loint(big) - (below ? 1 : 0);
 }
+// Within that band the offset is rounding, and its sign and its being zero
+// decide weights and gradients: it is formed as build_map_fast forms it.
 __device__ __forceinline__ int lean_element_exact(const Geom& g, const MapConst& mc, int d, double c, double& off) {
   const int i = axis_element_fast(g, mc, d, c);
-  off = c * mc.NL[d] - (double)i;
+  off = (c - g.h[d] * (double)i) * mc.invh[d];
   return i;
 }
+
+// Offset from a node (in cells) up to which a sampled point takes the general
+// path: above the FP32 rounding of an offset in [0, 1].
+constexpr double kLeanNodeBand = 1e-7;
 
 // Builds the compact map (3D) with the decisions of build_map_fast and
 // build_map_f32. Returns -1 outside the domain, 0 without triplets, 1
 // otherwise, 2 for the two rare cases the compact form does not hold: an
 // upper corner on the domain's upper face (it has no element) and a sampled
-// point on a node (its gradient is 0/0).
+// point on a node or within rounding of one (its gradient is 0/0 or, by the
+// offset's sign, jumps between -1/h and 1/h or falls away).
 template <typename R>
 __device__ __forceinline__ int lean_map(const Geom& g, const MapConst& mc, int cpdi_spec, const double* x, R extent,
                                         R sG, LeanMap<R>& lm, int* err) {
@@ -301,9 +308,8 @@ __device__ __forceinline__ int lean_map(const Geom& g, const MapConst& mc, int c
       atomicOr(err, kErrElemAlias);
       return 0;
     }
-    const R r = (R)off;
-    on_node = on_node || !(r > R(0) && r < R(1));
-    lm.a[d] = R(1) - r;
+    on_node = on_node || !(off > kLeanNodeBand && off < 1.0 - kLeanNodeBand);
+    lm.a[d] = R(1) - (R)off;
     lm.b[d] = sizeof(R) == 8 ? (R)-mc.invh[d] : (R)-mc.invhf[d];
   }
   lm.sS = R(1);

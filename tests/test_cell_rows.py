@@ -94,3 +94,43 @@ def test_cell_sums_mixed(name, kernel):
     for f in ("x", "x_t", "T"):
         assert_close(gpu.points(0, f), ref.points(0, f), 1e-4, f"{name} {f}", field_floor(case, f))
     gpu.close()
+
+
+def _on_nodes(nodes, cpdi):
+    """A body on a 20^3 grid whose h has no exact binary form: a cloud, and in
+    it points whose x coordinate (cpdi 0) or lower corner in x (cpdi 1) is
+    h * i, which is on node i up to the rounding of the product."""
+    n, h = 20, 1.0 / 20
+    vol = (h / 2) ** 3
+    half = 0.25 * np.cbrt(vol)
+    rng = np.random.default_rng(21)
+    x = rng.uniform(0.11, 0.89, (2000, 3))
+    for k, i in enumerate(nodes):
+        x[8 * k:8 * k + 8, 0] = h * i + (half if cpdi else 0.0)
+    x_t = (x - 0.5) @ np.array([[0.3, -1.0, 0.2], [1.0, -0.2, 0.5], [-0.4, 0.1, 0.6]])
+    body = inputs.Body("nodes", np.full(2000, 1000.0 * vol), np.full(2000, vol), x, x_t, np.ones(2000, np.int32), E=1e4)
+    return inputs.Case("nodes", 3, (1.0,) * 3, (n,) * 3, 1e-5, 8, [body], cpdi=cpdi)
+
+
+# The offset of such a point from its node is rounding, and the sampled map's
+# gradient follows its sign (1/h or -1/h) and is 0/0 where it is zero: both
+# kernel forms must take it alike. Formed as (x - h i) / h it is zero at nodes
+# 4, 8 and 16 and negative at 9, 13 and 18; formed as x N / L - i it is positive
+# at all six. The same nodal sums in another order: 1e-10 in FP64, 1e-4 in the
+# mixed form.
+@pytest.mark.parametrize("mode,tol", [("fp64", FP64_TOL), ("mixed", 1e-4)])
+@pytest.mark.parametrize("nodes,cpdi", [((9, 13, 18), 0), ((4, 8, 16), 0), ((5, 10, 15), 0),
+                                        ((4, 5, 8, 9, 10, 13, 15, 16), 1)])
+def test_points_on_nodes_as_in_the_staged_kernel(nodes, cpdi, mode, tol):
+    case = _on_nodes(nodes, cpdi)
+    runs = []
+    for kernel in (("staged", 512), ("point_per_thread", 512), ("point_per_thread", 128)):
+        gpu = GPUExplicitUSL(case, mode=mode, kernel=kernel)
+        gpu.step(1)
+        runs.append(([gpu.points(0, f) for f in ("x", "x_t", "v", "T")], gpu.active_nodes()[0]))
+        gpu.close()
+    for got, active in runs[1:]:
+        assert active == runs[0][1], "nodes with mass"
+        for f, g, r in zip(("x", "x_t", "v", "T"), got, runs[0][0]):
+            assert np.array_equal(np.isnan(g), np.isnan(r)), f"{f}: NaN at other points"
+            assert_close(np.nan_to_num(g), np.nan_to_num(r), tol, f, field_floor(case, f))
