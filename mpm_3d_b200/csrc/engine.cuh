@@ -37,8 +37,10 @@
 #include "../../include/mpm_b200.h"
 #include "fused.cuh"
 #include "frame.cuh"
+#include "fused_kernels.cuh"
 #include "fused_lean.cuh"
 #include "kernels_fp64.cuh"
+#include "material.cuh"
 #include "sort.cuh"
 
 namespace mpmb200 {
@@ -2173,8 +2175,12 @@ class Batch : public BatchBase {
 
   int stride_blocks(int threads) const { return sm_count_ * (2048 / threads); }
 
-  template <int DIM, int CAP, bool NORMAL, bool SINGLE, bool DET>
-  mpmgpu_status launch_fused_k(int prime_pass, int phases, int one_body, cudaStream_t st) {
+  // One launch of the fused kernel: over body one_body (its parameters then
+  // sit in the constant bank), or over the table (-1). `per_sm` is the
+  // kernel's entry in the table of resident CTAs per SM, looked up once per
+  // kernel (before any capture).
+  mpmgpu_status launch_kernel(const FusedKernel& k, int& per_sm, const char* name, int prime_pass, int phases,
+                              int one_body, cudaStream_t st) {
     FusedLaunch<PT> fl{};
     if (publish_ && !prime_pass) {
       fl.active_acc = active_acc_;
@@ -2182,8 +2188,8 @@ class Batch : public BatchBase {
       fl.blocks = count_;
       publish_ = false;
     }
-    if (SINGLE) fl.one = ctx_host_[(size_t)one_body];
-    fl.one_body = SINGLE ? one_body : -1;
+    if (one_body >= 0) fl.one = ctx_host_[(size_t)one_body];
+    fl.one_body = one_body;
     fl.bodies = ctx_d_;
     fl.item_off = item_off_d_;
     fl.nwork_body = nwork_body_;
@@ -2202,96 +2208,64 @@ class Batch : public BatchBase {
     fl.bounds = bounds_;
     fl.wait_polls = wait_polls_;
     fl.queue = queue_;
-    constexpr size_t smem = fused_smem_bytes<DIM, PT, CAP, NORMAL, DET>();
-    auto kern = k_g2p2g<DIM, PT, CAP, NORMAL, SINGLE, DET>;
-    // resident CTAs per SM, looked up once per kernel (before any capture)
-    int& per_sm = fused_per_sm_[((CAP == 256 ? 0 : (CAP == 512 ? 1 : 2)) * 4 + (NORMAL ? 2 : 0) + (SINGLE ? 1 : 0)) * 2 +
-                                (DET ? 1 : 0)];
     if (per_sm == 0) {
-      MPM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      MPM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, fused_threads<PT, CAP>(), smem));
+      MPM_CUDA_TRY(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem));
+      MPM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, k.threads, k.smem));
       if (per_sm < 1) return fail(MPMGPU_ERR_CUDA, "fused kernel does not fit on an SM");
     }
-    const int blocks = per_sm * sm_count_;
     StageTimer timer(this, kStageFused);
-    kern<<<blocks, fused_threads<PT, CAP>(), smem, st>>>(fl);
-    return check_launch("k_g2p2g");
-  }
-
-  // One launch per body for small batches at the default item size (the
-  // body's parameters then sit in the constant bank), else one launch per
-  // kind of body (with or without the contact normal) over the table.
-  template <int DIM, int CAP, bool DET>
-  mpmgpu_status launch_fused_t(int prime_pass, int phases) {
-    if constexpr (CAP == 512) {
-      if (single_mode_) {
-        return one_body_launches(prime_pass, [&](int b, cudaStream_t st) {
-          if (ctx_host_[(size_t)b].needs_normal) return launch_fused_k<DIM, CAP, true, true, DET>(prime_pass, phases, b, st);
-          return launch_fused_k<DIM, CAP, false, true, DET>(prime_pass, phases, b, st);
-        });
-      }
+    void* args[] = {&fl};
+    const cudaError_t e = cudaLaunchKernel(k.fn, dim3((unsigned)(per_sm * sm_count_)), dim3((unsigned)k.threads), args,
+                                           k.smem, st);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return fail(MPMGPU_ERR_CUDA, std::string(name) + ": " + cudaGetErrorString(e));
     }
-    if (any_plain_) MPM_TRY((launch_fused_k<DIM, CAP, false, false, DET>(prime_pass, phases, -1, stream_)));
-    if (any_normal_) MPM_TRY((launch_fused_k<DIM, CAP, true, false, DET>(prime_pass, phases, -1, stream_)));
+    launches_++;
     return MPMGPU_OK;
   }
 
-  template <int NT, int PPT, bool NORMAL, bool SINGLE, int MAT>
-  mpmgpu_status launch_lean_k(int prime_pass, int phases, int one_body, cudaStream_t st) {
-    FusedLaunch<PT> fl{};
-    if (publish_ && !prime_pass) {
-      fl.active_acc = active_acc_;
-      fl.active_pub = active_nodes_;
-      fl.blocks = count_;
-      publish_ = false;
-    }
-    if (SINGLE) fl.one = ctx_host_[(size_t)one_body];
-    fl.one_body = SINGLE ? one_body : -1;
-    fl.bodies = ctx_d_;
-    fl.item_off = item_off_d_;
-    fl.nwork_body = nwork_body_;
-    fl.work_end_body = work_end_body_;
-    fl.flat_body = flat_body_;
-    fl.flat_item = flat_item_;
-    fl.nbodies_cap = (int)ctx_host_.size();
-    fl.work_bin = work_bin_;
-    fl.work_start = work_start_;
-    fl.work_end = work_end_;
-    fl.nwork = nwork_;
-    fl.err = err_;
-    fl.drift = drift_;
-    fl.prime_pass = prime_pass;
-    fl.phases = phases;
-    fl.bounds = nullptr;
-    fl.wait_polls = wait_polls_;
-    fl.queue = queue_;
-    constexpr size_t smem = lean_smem_bytes<3, PT, NT * PPT>();
-    auto kern = k_g2p2g_lean<3, PT, NT, PPT, NORMAL, SINGLE, MAT>;
-    int& per_sm =
-        lean_per_sm_[(PPT == 2 ? 16 : 0) + (NT == 128 ? 8 : 0) + (NORMAL ? 4 : 0) + (SINGLE ? 2 : 0) + (MAT == 0 ? 1 : 0)];
-    if (per_sm == 0) {
-      MPM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      MPM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem));
-      if (per_sm < 1) return fail(MPMGPU_ERR_CUDA, "fused kernel does not fit on an SM");
-    }
-    StageTimer timer(this, kStageFused);
-    kern<<<per_sm * sm_count_, NT, smem, st>>>(fl);
-    return check_launch("k_g2p2g_lean");
+  // The staged kernel. One launch per body for small batches at the default
+  // item size (launch_kernel), else one launch per kind of body (with or
+  // without the contact normal) over the table.
+  mpmgpu_status launch_staged(int prime_pass, int phases) {
+    auto launch = [&](bool normal, int one_body, cudaStream_t st) {
+      const bool single = one_body >= 0;
+      FusedKernel k;
+      if constexpr (sizeof(PT) == 8)
+        k = det_ ? staged_kernel<PT, true>(dim_, cap_, normal, single) : staged_kernel<PT, false>(dim_, cap_, normal, single);
+      else
+        k = staged_kernel<PT, false>(dim_, cap_, normal, single);
+      int& per_sm = fused_per_sm_[((cap_ == 256 ? 0 : (cap_ == 512 ? 1 : 2)) * 2 + (normal ? 1 : 0)) * 2 + (single ? 1 : 0)];
+      return launch_kernel(k, per_sm, "k_g2p2g", prime_pass, phases, one_body, st);
+    };
+    if (cap_ == 512 && single_mode_)
+      return one_body_launches(
+          prime_pass, [&](int b, cudaStream_t st) { return launch(ctx_host_[(size_t)b].needs_normal != 0, b, st); });
+    if (any_plain_) MPM_TRY(launch(false, -1, stream_));
+    if (any_normal_) MPM_TRY(launch(true, -1, stream_));
+    return MPMGPU_OK;
   }
 
-  template <int NT, int PPT, bool NORMAL, bool SINGLE>
-  mpmgpu_status launch_lean_s(int prime_pass, int phases, int one_body, bool elastic, cudaStream_t st) {
-    if (elastic) return launch_lean_k<NT, PPT, NORMAL, SINGLE, 0>(prime_pass, phases, one_body, st);
-    return launch_lean_k<NT, PPT, NORMAL, SINGLE, -1>(prime_pass, phases, one_body, st);
-  }
-
-  // points per item: 128 (CTAs of 128 threads), 256 (256 threads) or 512
-  // (256 threads, two points each)
-  template <bool NORMAL, bool SINGLE>
-  mpmgpu_status launch_lean_m(int prime_pass, int phases, int one_body, bool elastic, cudaStream_t st) {
-    if (cap_ == 128) return launch_lean_s<128, 1, NORMAL, SINGLE>(prime_pass, phases, one_body, elastic, st);
-    if (cap_ == 512) return launch_lean_s<256, 2, NORMAL, SINGLE>(prime_pass, phases, one_body, elastic, st);
-    return launch_lean_s<256, 1, NORMAL, SINGLE>(prime_pass, phases, one_body, elastic, st);
+  // The point-per-thread kernel, launched the same way at every item size.
+  mpmgpu_status launch_lean(int prime_pass, int phases) {
+    auto launch = [&](bool normal, int one_body, bool elastic, cudaStream_t st) {
+      const bool single = one_body >= 0;
+      const FusedKernel k = cap_ == 128   ? lean_kernel<PT, 128>(normal, single, elastic)
+                            : cap_ == 512 ? lean_kernel<PT, 512>(normal, single, elastic)
+                                          : lean_kernel<PT, 256>(normal, single, elastic);
+      int& per_sm = lean_per_sm_[((cap_ == 128 ? 0 : (cap_ == 512 ? 2 : 1)) * 2 + (normal ? 1 : 0)) * 4 +
+                                 (single ? 2 : 0) + (elastic ? 1 : 0)];
+      return launch_kernel(k, per_sm, "k_g2p2g_lean", prime_pass, phases, one_body, st);
+    };
+    if (single_mode_)
+      return one_body_launches(prime_pass, [&](int b, cudaStream_t st) {
+        const BodyCtx<PT>& c = ctx_host_[(size_t)b];
+        return launch(c.needs_normal != 0, b, !c.mat.has_material || c.mat.kind == 0, st);
+      });
+    if (any_plain_) MPM_TRY(launch(false, -1, all_elastic_, stream_));
+    if (any_normal_) MPM_TRY(launch(true, -1, all_elastic_, stream_));
+    return MPMGPU_OK;
   }
 
   // The one-body launches of a stage, body by body (bodies still to prime
@@ -2331,37 +2305,8 @@ class Batch : public BatchBase {
     return MPMGPU_OK;
   }
 
-  mpmgpu_status launch_lean(int prime_pass, int phases) {
-    if (single_mode_) {
-      return one_body_launches(prime_pass, [&](int b, cudaStream_t st) {
-        const BodyCtx<PT>& c = ctx_host_[(size_t)b];
-        const bool el = !c.mat.has_material || c.mat.kind == 0;
-        if (c.needs_normal) return launch_lean_m<true, true>(prime_pass, phases, b, el, st);
-        return launch_lean_m<false, true>(prime_pass, phases, b, el, st);
-      });
-    }
-    if (any_plain_) MPM_TRY((launch_lean_m<false, false>(prime_pass, phases, -1, all_elastic_, stream_)));
-    if (any_normal_) MPM_TRY((launch_lean_m<true, false>(prime_pass, phases, -1, all_elastic_, stream_)));
-    return MPMGPU_OK;
-  }
-
   mpmgpu_status launch_fused(int prime_pass, int phases) {
-    if (form_ != kFormStaged) return launch_lean(prime_pass, phases);
-    if constexpr (sizeof(PT) == 8) {
-      if (det_) {
-        // the deterministic form: 256 points per item in 3D (two tile levels)
-        if (dim_ == 3) return launch_fused_t<3, 256, true>(prime_pass, phases);
-        return launch_fused_t<2, 512, true>(prime_pass, phases);
-      }
-    }
-    if (dim_ == 3) {
-      if (cap_ == 256) return launch_fused_t<3, 256, false>(prime_pass, phases);
-      if constexpr (sizeof(PT) == 4) {
-        if (cap_ == 1024) return launch_fused_t<3, 1024, false>(prime_pass, phases);
-      }
-      return launch_fused_t<3, 512, false>(prime_pass, phases);
-    }
-    return launch_fused_t<2, 512, false>(prime_pass, phases);
+    return form_ == kFormStaged ? launch_staged(prime_pass, phases) : launch_lean(prime_pass, phases);
   }
 
   // Deterministic form: per-body bounds of the nodal contributions from the
@@ -2623,7 +2568,7 @@ class Batch : public BatchBase {
   int cap_ = 512;
   bool cap_auto_ = false, sort_auto_ = false;   // chosen by the defaults' rules, not by the caller
   int sm_count_ = 148;
-  int fused_per_sm_[24] = {};
+  int fused_per_sm_[12] = {};
   cudaStream_t copy_stream_ = nullptr;
   cudaEvent_t upload_ev_ = nullptr;
   // one-body launches of the second to fourth body (one_body_launches)
@@ -2676,7 +2621,7 @@ class Batch : public BatchBase {
   bool all_elastic_ = true;              // every body IsotropicLinearElasticity (or no material)
   int form_ = kFormStaged;               // form of the fused kernel (cap_: its points per item)
   uint32_t wait_polls_ = kWaitPolls;     // poll limit of the fused kernels' first waits
-  int lean_per_sm_[32] = {};
+  int lean_per_sm_[24] = {};
   int flip_ = 0;                        // point buffers swapped an odd number of times
   cudaStream_t stream_ = nullptr;
   std::vector<HJob> jobs_;

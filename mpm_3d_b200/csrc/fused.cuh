@@ -32,8 +32,7 @@
 
 #include "async_copy.cuh"
 #include "geom.cuh"
-#include "kernels_fp64.cuh"
-#include "sort.cuh"
+#include "material.cuh"
 #include "state.cuh"
 
 namespace mpmb200 {

@@ -132,6 +132,40 @@ struct GridBody {
   double mu_f;       // CartesianFrictionalBox friction
 };
 
+// Bin layout for a grid.
+struct BinGeom {
+  int B;             // cells per bin per axis (4 in 3D, 8 in 2D)
+  int cells_per_bin; // B^dim (64)
+  int nbx, nby, nbz; // bins per axis
+  int nbins;         // total bins (the inactive points use key nbins)
+  int T;             // tile nodes per axis, B + 3
+  int tile_nodes;    // T^dim
+};
+
+// Per-body table entry. The first part (up to Palt) is what the fused
+// kernel stages in shared memory for a work item.
+template <typename PT>
+struct alignas(16) BodyCtx {
+  Geom g;
+  MapConst mc;
+  BinGeom bg;
+  StepParams sp;
+  MaterialParams mat;
+  PointsT<PT> P;        // current storage order
+  NodesVel V;
+  NodesAcc A;
+  NodesAcc Ar;          // deterministic form: level-1 (remainder) sums, else null
+  uint32_t* flags;      // node-block flags of the body's job (its first block)
+  int needs_normal;     // accumulate the contact normal (first body of a contact)
+  int prime;            // 1 until the body's first scatter has run
+  // sort side
+  PointsT<PT> Palt;     // second buffer; swapped with P after a sort
+  int64_t point_off;    // first point in the batch's point space
+  int64_t bin_off;      // first entry in the batch's bin arrays (nbins + 1 per body)
+  int64_t cell_off;     // first cell counter (nbins * cells_per_bin + 1 per body)
+  int inst;
+};
+
 // Sizes of the batch's index spaces, read by the kernels on the device so
 // that captured graphs stay valid while jobs come and go.
 struct BatchHdr {
