@@ -397,18 +397,19 @@ __device__ __forceinline__ GatherSum<R> gather_box_any(const PointMapT<R>& pm, c
   return gather_rolled<DIM, T, TN>(pm, o, tvel, mask);
 }
 
-// Gather over any window (three-node spans, nodes outside the tile).
-template <int DIM, int T, int TN, typename PT, typename R>
+// Gather over any window (three-node spans, nodes outside the tile). TILED =
+// false: every node from global memory, and no drift counted.
+template <int DIM, int T, int TN, bool TILED = true, typename PT, typename R>
 __device__ __forceinline__ GatherSum<R> gather_general(const BodyCtx<PT>& c, unsigned long long* drift,
                                                        const PointMapT<R>& pm, const int* o, const R* tvel,
                                                        const double* vref) {
   GatherSum<R> gs;
   const Geom& g = c.g;
-  const bool in_tile = window_in_tile<DIM>(pm, o, T);
-  if (!in_tile) atomicAdd(drift, 1ull);
+  const bool in_tile = TILED && window_in_tile<DIM>(pm, o, T);
+  if (TILED && !in_tile) atomicAdd(drift, 1ull);
   using TL = TileLayout<DIM, T>;
-  const int txy = (pm.ax[0].base - o[0]) + TL::RL * (pm.ax[1].base - o[1]);
-  const int bz = DIM == 3 ? pm.ax[2].base - o[2] : 0;
+  const int txy = !TILED ? 0 : (pm.ax[0].base - o[0]) + TL::RL * (pm.ax[1].base - o[1]);
+  const int bz = TILED && DIM == 3 ? pm.ax[2].base - o[2] : 0;
   const R sS = pm.sS, sG = pm.sG;
   for_window<DIM>(pm, [&](int k0, int k1, int k2) {
     const R wz = DIM == 3 ? sel3(pm.ax[2].W, k2) : R(1);
@@ -769,20 +770,20 @@ __device__ __forceinline__ void scatter_box_any(const PointMapT<R>& pm, const in
 }
 
 // Scatter over any window (three-node spans, nodes outside the tile, which
-// go straight to the global accumulators).
-template <int DIM, int T, int TN, bool NORMAL, bool DET, typename PT, typename R>
+// go straight to the global accumulators; TILED = false: all, none counted).
+template <int DIM, int T, int TN, bool NORMAL, bool DET, bool TILED = true, typename PT, typename R>
 __device__ __forceinline__ void scatter_general(const BodyCtx<PT>& c, unsigned long long* drift,
                                                 const PointMapT<R>& pm, const int* o, const ScatterSrc<R>& q,
                                                 double* tacc, uint8_t* touched, const Split2* ks) {
   const Geom& g = c.g;
-  const bool in_tile = window_in_tile<DIM>(pm, o, T);
+  const bool in_tile = TILED && window_in_tile<DIM>(pm, o, T);
   if (!in_tile) {
-    atomicAdd(drift, 1ull);
+    if (TILED) atomicAdd(drift, 1ull);
     mark_blocks<DIM>(g, pm, c.flags);
   }
   using TL = TileLayout<DIM, T>;
-  const int txy = (pm.ax[0].base - o[0]) + TL::RL * (pm.ax[1].base - o[1]);
-  const int bz = DIM == 3 ? pm.ax[2].base - o[2] : 0;
+  const int txy = !TILED ? 0 : (pm.ax[0].base - o[0]) + TL::RL * (pm.ax[1].base - o[1]);
+  const int bz = TILED && DIM == 3 ? pm.ax[2].base - o[2] : 0;
   const R sS = pm.sS, sG = pm.sG;
   for_window<DIM>(pm, [&](int k0, int k1, int k2) {
     const R wz = DIM == 3 ? sel3(pm.ax[2].W, k2) : R(1);

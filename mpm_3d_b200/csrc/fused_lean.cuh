@@ -474,13 +474,14 @@ __device__ __forceinline__ void lean_update(const BodyCtx<PT>& c, int64_t p, con
   }
 }
 
-// One point of the far list, node by node from and to global memory.
+// One point of the far list, node by node from and to global memory. A visit
+// counts as drift where the window is outside the item's tile (origin o), not
+// where only the compact map does not hold it.
 template <bool NORMAL, int MAT, typename PT>
 __device__ __forceinline__ void lean_far_point(const BodyCtx<PT>& c, int* err, unsigned long long* drift, int64_t p,
-                                               bool whole, const double* vref, int stepping) {
+                                               bool whole, const int* o, const double* vref, int stepping) {
   using R = PT;
   const PointsT<PT>& P = c.P;
-  const int o[3] = {1 << 29, 1 << 29, 1 << 29};   // no node is in the tile
   const R ext = P.ext[p];
   double x[3], vd[3];
   R s6[6];
@@ -495,7 +496,8 @@ __device__ __forceinline__ void lean_far_point(const BodyCtx<PT>& c, int* err, u
   if (whole) {
     GatherSum<R> gs;
     if (build_map<3>(c.g, c.mc, c.sp.cpdi, x, ext, pm, err) > 0) {
-      gs = gather_general<3, kLeanSide + 1, 1>(c, drift, pm, o, (const R*)nullptr, vref);
+      if (!window_in_tile<3>(pm, o, kLeanSide + 1)) atomicAdd(drift, 1ull);
+      gs = gather_general<3, kLeanSide + 1, 1, false>(c, drift, pm, nullptr, (const R*)nullptr, vref);
       if constexpr (sizeof(PT) == 4) add_reference<3>(pm, vref, gs);
     }
     const R u[3] = {P.u[0][p], P.u[1][p], P.u[2][p]};
@@ -516,7 +518,9 @@ __device__ __forceinline__ void lean_far_point(const BodyCtx<PT>& c, int* err, u
   for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int k = 0; k < 3; k++) q.V3[i][k] = V3[i][k];
-  scatter_general<3, kLeanSide + 1, 1, NORMAL, false>(c, drift, pm, o, q, (double*)nullptr, (uint8_t*)nullptr, nullptr);
+  if (!window_in_tile<3>(pm, o, kLeanSide + 1)) atomicAdd(drift, 1ull);
+  scatter_general<3, kLeanSide + 1, 1, NORMAL, false, false>(c, drift, pm, nullptr, q, (double*)nullptr,
+                                                             (uint8_t*)nullptr, nullptr);
 }
 
 // One point from gather to its record. `a` is its active state (1 active, 2
@@ -1035,7 +1039,10 @@ __global__ void __launch_bounds__(NT, lean_min_ctas<PT, NT, PPT>())
     const int nfar = (int)sh.mask[kLeanMask];
     for (int t = threadIdx.x; t < nfar; t += NT) {
       const int f = sh.far[t];
-      lean_far_point<NORMAL, MAT>(c, fl.err, fl.drift, pstart + (f & 511), f < kFarScatter, vref, prime ? 0 : 1);
+      int fo[3];   // o, formed again: held through the row sums it costs 10 us of the column's step
+      bin_origin(c, bin, fo);
+      lean_far_point<NORMAL, MAT>(c, fl.err, fl.drift, pstart + (f & 511), f < kFarScatter, fo, vref,
+                                  prime ? 0 : 1);
     }
     advance();
     __syncthreads();

@@ -134,3 +134,18 @@ def test_points_on_nodes_as_in_the_staged_kernel(nodes, cpdi, mode, tol):
         for f, g, r in zip(("x", "x_t", "v", "T"), got, runs[0][0]):
             assert np.array_equal(np.isnan(g), np.isnan(r)), f"{f}: NaN at other points"
             assert_close(np.nan_to_num(g), np.nan_to_num(r), tol, f, field_floor(case, f))
+
+
+@pytest.mark.parametrize("name", sorted(CLOUDS))
+def test_drift_is_counted_as_in_the_staged_kernel(name):
+    """mpmgpu_active_nodes: visits that found a point outside its bin's tile.
+    Points that take the general path for another reason (corners on the upper
+    face) are none, and the two kernel forms share the bins."""
+    counts = []
+    for kernel in (("staged", 512), ("point_per_thread", 512), ("point_per_thread", 128)):
+        gpu = GPUExplicitUSL(CLOUDS[name](), kernel=kernel)
+        gpu.step(6)
+        counts.append(gpu.active_nodes()[1])
+        gpu.close()
+    assert counts[1:] == counts[:1] * 2
+    assert (counts[0] > 0) == name.startswith("drift")
