@@ -294,10 +294,12 @@ typedef enum {
   MPMGPU_KERNEL_POINT_PER_THREAD = 1
 } mpmgpu_kernel_form;
 
-/* Selects the fused kernel's form and points per work item (default: one
- * point per thread in 3D outside the deterministic form, with 512 points, or
- * 128 for jobs of up to 65,536 points in all, else staged with 512); MPMGPU_ERR_ARG if the pair is not available for
- * the handle. Takes effect at the next step. */
+/* Selects the fused kernel's form and points per work item; MPMGPU_ERR_ARG if
+ * the pair is not available for the handle. Takes effect at the next step.
+ * Default in 3D outside the deterministic form: one point per thread, with 128
+ * points per item for jobs of up to 65,536 points in all or of up to two points
+ * per grid cell they fill, else 512. Else: staged with 512 (256 in 3D).
+ * mpmgpu_kernel reports what the next step runs. */
 mpmgpu_status mpmgpu_set_kernel(mpmgpu_handle* h, int form, int points_per_item);
 mpmgpu_status mpmgpu_kernel(const mpmgpu_handle* h, int* form, int* points_per_item);
 /* No counterpart in the reference. Tunes the handle's launch shape on its
@@ -346,10 +348,10 @@ typedef struct {
   int sort_interval;   /* steps between re-binnings (0 = default: 32 with up
                           to four bodies in the batch, 16 with more) */
   int points_per_item; /* points per CTA work item: 0 = default (3D,
-                          not deterministic: 512 on the point-per-thread
-                          kernel, 128 while the jobs have up to 65,536
-                          points in all; else 512 on the staged kernel); 128, 256
-                          or 512 run on the point-per-thread kernel where
+                          not deterministic: 128 or 512 on the
+                          point-per-thread kernel, by the points of the
+                          stepped jobs, see mpmgpu_set_kernel; else 512 on
+                          the staged kernel, 256 in 3D); 128, 256 or 512 run on the point-per-thread kernel where
                           it applies, other sizes on the staged kernel
                           (1024 in the 3D mixed form, 512 in 2D); see
                           mpmgpu_set_kernel and mpmgpu_batch_autotune */

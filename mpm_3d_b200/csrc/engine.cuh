@@ -152,6 +152,18 @@ inline bool cap_available(int dim, bool mixed, int cap) {
 // of 96,000 points 28.5 -> 32.7, 128,000 sand points 32.8 -> 40.6.
 constexpr int64_t kSmallPoints = 65536;
 
+// Above that they follow the points of a filled bin (64 cells), estimated from
+// the bodies' volumes, 2 % allowed for rounding: an item never spans bins, so
+// where a bin holds 128 points or fewer a CTA of 256 threads is mostly idle
+// (bodies of one point per cell had become 3 to 10 % slower than with the
+// kernel that added into shared tiles). Measured (us per step at 128 / 256 /
+// 512 points): one point per cell, 373,000 points on a lattice FP64 142 / 191 /
+// 203, mixed 146 / 177 / 187, at random 257 / 365 / 349 and 248 / 320 / 321; two
+// per cell, 746,000 points 158 / 217 / 216 and 165 / 191 / 200; three per cell,
+// 1.1 M points 319 / 294 / 288 and 319 / 265 / 264, at random 480 / 528 / 497 and
+// 467 / 443 / 456; eight per cell, 3 M points 502 / 474 / 365 and 532 / 419 / 337.
+inline int items_for_bin(double points_per_bin) { return points_per_bin <= 1.02 * 128 ? 128 : 512; }
+
 // Default steps between re-binnings: 32 for up to four bodies, 16 for more
 // (launches over the body table), whose jobs move at unlike speeds and are
 // re-binned together. A point that has drifted out of its item's tile takes
@@ -348,9 +360,9 @@ class BatchBase {
   virtual int points_per_item() const = 0;
   virtual int sort_interval() const = 0;
   // Form of the fused kernel (kFormStaged, kFormLean) and
-  // its points per work item; chosen at creation (the point-per-thread
-  // kernel with 512 points in 3D, the staged kernel otherwise), by the
-  // autotuner, or by set_kernel.
+  // its points per work item; chosen by the defaults (the point-per-thread
+  // kernel in 3D, its size by the points of the stepped jobs; the staged
+  // kernel otherwise), by the autotuner, or by set_kernel.
   virtual int kernel_form() const = 0;
   virtual mpmgpu_status set_kernel(int form, int cap) = 0;
   virtual mpmgpu_status active_nodes(int64_t* nodes, int64_t* drifted) = 0;
@@ -373,6 +385,7 @@ class Batch : public BatchBase {
     double mu_f = 0.0;
     int needs_normal = 0;
     int prime = 1;
+    double cells = 0.0;   // grid cells its points' volumes fill
     std::vector<void*> allocs;
   };
   struct HJob {
@@ -479,7 +492,20 @@ class Batch : public BatchBase {
   bool mixed() const override { return sizeof(PT) == 4; }
   cudaStream_t stream() const override { return stream_; }
   int64_t launches() const override { return launches_; }
-  int points_per_item() const override { return cap_; }
+  int points_per_item() const override {
+    if (!cap_auto_ || form_ != kFormLean) return cap_;
+    // as the next step's commit will have it
+    int64_t points = 0;
+    double cells = 0.0;
+    for (const auto& j : jobs_) {
+      if (j.removed || j.finished || j.steps_left <= 0) continue;
+      for (const auto& b : j.bodies) {
+        points += b.n;
+        cells += b.cells;
+      }
+    }
+    return points > 0 ? auto_cap(points, cells) : cap_;
+  }
 
   // Nodes with mass (per body) in the last step's grid update, and points
   // found outside their bin's tile since the batch was created.
@@ -609,6 +635,10 @@ class Batch : public BatchBase {
         for (int64_t i = a; i < b; i++) h[i] = (int32_t)i;
       }));
     }
+    double vol_sum = 0.0, cell = 1.0;
+    for (int64_t i = 0; i < n; i++) vol_sum += desc.v[i];
+    for (int d = 0; d < D; d++) cell *= j->g.h[d];
+    B.cells = vol_sum / cell;
     B.mat = make_material(desc.has_material, desc.E, desc.nu, desc.material_kind, desc.material_props,
                           desc.material_flags);
     B.has_boundary = desc.has_boundary;
@@ -1819,6 +1849,11 @@ class Batch : public BatchBase {
     return MPMGPU_OK;
   }
 
+  // Points per item of the point-per-thread kernel by default, for `points` in
+  // bodies that fill `cells` grid cells.
+  int auto_cap(int64_t points, double cells) const {
+    return points <= kSmallPoints ? 128 : items_for_bin(64.0 * (double)points / cells);
+  }
   int default_cap() const { return det_ && dim_ == 3 ? 256 : 512; }
 
   // Converts block-linear nodal arrays (comps SoA components, host copies)
@@ -1975,6 +2010,7 @@ class Batch : public BatchBase {
     std::vector<int64_t> point_end, bin_end;
     std::vector<int32_t> item_off;
     int64_t points = 0, bins = 0, cells = 0, items = 0;
+    double filled = 0.0;   // grid cells the bodies fill
     live_jobs_ = 0;
     bool any_prime = false;
     for (auto& j : jobs_) {
@@ -2024,6 +2060,7 @@ class Batch : public BatchBase {
         c.cell_off = cells;
         c.inst = j.slot;
         points += b.n;
+        filled += b.cells;
         bins += j.bg.nbins + 1;
         cells += (int64_t)j.bg.nbins * j.bg.cells_per_bin + 1;
         item_off.push_back((int32_t)items);
@@ -2071,7 +2108,7 @@ class Batch : public BatchBase {
     single_mode_ = ctx.size() <= (size_t)kSideStreams + 1;   // one launch per body, concurrent (one_body_launches)
     // the defaults follow the jobs (the work list is rebuilt below whenever
     // the membership changes)
-    if (membership && cap_auto_ && form_ == kFormLean) cap_ = points <= kSmallPoints ? 128 : kDefaultLeanCap;
+    if (membership && cap_auto_ && form_ == kFormLean) cap_ = auto_cap(points, filled);
     if (sort_auto_) sort_interval_ = single_mode_ ? kSortInterval : kSortIntervalTable;
     any_plain_ = any_normal_ = false;
     all_elastic_ = true;

@@ -184,3 +184,53 @@ def test_mixed_sand_within_1e4_of_fp64():
     columns, with their elastic, plastic-return and zero-stress points."""
     for c in (inputs.sand_column(2, steps=80), inputs.sand_column(3, n_cells=12, steps=30)):
         _compare(c, _solo(c, c.steps, mode="mixed"), _solo(c, c.steps), MIXED_TOL, f"mixed {c.name}")
+
+
+def _block(n, side, per_cell):
+    """A cube of `side` cells per axis on an n^3 grid with per_cell[d] points
+    per cell and axis."""
+    h = 1.0 / n
+    ax = [(0.25 * n // 1 + (np.arange(side * p) + 0.5) / p) * h for p in per_cell]
+    x = np.stack(np.meshgrid(*ax, indexing="ij"), -1).reshape(-1, 3)
+    vol = h ** 3 / np.prod(per_cell)
+    m = len(x)
+    v = (x - x.mean(0)) @ np.array([[0.1, -1.0, 0.2], [1.0, -0.1, 0.3], [-0.2, 0.1, 0.15]])
+    body = inputs.Body("block", np.full(m, 1000 * vol), np.full(m, vol), x, v, np.ones(m, np.int32))
+    return inputs.Case("block", 3, (1.0,) * 3, (n,) * 3, 1e-5, 6, [body])
+
+
+# 70,000 to 74,000 points each: a bin's 64 cells hold 64, 128, 256 or 512 points
+@pytest.mark.parametrize("per_cell,side,want", [((1, 1, 1), 42, 128), ((2, 1, 1), 33, 128), ((2, 2, 1), 26, 512),
+                                                ((2, 2, 2), 21, 512), ((2, 2, 2), 8, 128)])
+@pytest.mark.parametrize("mode", ["fp64", "mixed"])
+def test_default_item_size_follows_the_points_of_a_bin(per_cell, side, want, mode):
+    sim = GPUExplicitUSL(_block(64, side, per_cell), mode=mode)
+    assert sim.kernel() == ("point_per_thread", want)   # what the first step will run
+    sim.step(1)
+    assert sim.kernel() == ("point_per_thread", want)
+    sim.set_kernel("point_per_thread", 256)
+    sim.step(1)
+    assert sim.kernel() == ("point_per_thread", 256)    # the caller's choice stays
+    sim.close()
+
+
+def test_default_item_size_follows_jobs_that_join_and_leave():
+    """Jobs across the 65,536-point line in both directions: the work list is
+    cut anew each time, and every job computes what it computes alone."""
+    small = _block(24, 8, (2, 2, 2))
+    large = _block(64, 21, (2, 2, 2))
+    batch = GPUBatch(dim=3, mode="fp64")
+    a = batch.add(small, steps=30)
+    batch.step(4)
+    assert batch.points_per_item() == 128
+    b = batch.add(large, steps=6)
+    batch.step(3)
+    assert batch.points_per_item() == 512
+    batch.step(3)      # the large job has run its steps
+    assert batch.points_per_item() == 128
+    batch.step(20)
+    batch.synchronize()
+    assert batch.state(a) == (30, 0) and batch.state(b) == (6, 0)
+    _compare(small, _from_batch(batch, a, small), _solo(small, 30), FP64_TOL, "small job")
+    _compare(large, _from_batch(batch, b, large), _solo(large, 6), FP64_TOL, "large job")
+    batch.close()
