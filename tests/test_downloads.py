@@ -1,0 +1,47 @@
+"""Point read-back: several jobs' fields in one call equal each job's own, bit
+for bit, on every path (device conversion in one group, in several, and host
+conversion), with chunk and thread boundaries inside the jobs."""
+import os
+import threading
+
+import numpy as np
+import pytest
+
+from mpm_3d_b200 import inputs
+from mpm_3d_b200.native import POINT_FIELDS, GPUBatch, GPUExplicitUSL, MpmGpuError
+from util import bits_equal
+
+pytestmark = pytest.mark.gpu
+
+GENERAL = [f for f in POINT_FIELDS if f not in ("L", "gammap", "gammap_dot")]
+
+
+def _cloud(dim, n_points, seed, material="IsotropicLinearElasticity"):
+    """n_points points at random in the inner part of a 48^dim grid."""
+    rng = np.random.default_rng(seed)
+    x, v = np.zeros((n_points, 3)), np.zeros((n_points, 3))
+    x[:, :dim] = rng.uniform(0.2, 0.8, (n_points, dim))
+    v[:, :dim] = rng.uniform(-1.0, 1.0, (n_points, dim))
+    vol = (1.0 / 96) ** dim
+    body = inputs.Body("cloud", np.full(n_points, 1000 * vol), np.full(n_points, vol), x, v,
+                       np.ones(n_points, np.int32), material_class=material)
+    return inputs.Case("cloud", dim, (1.0,) * dim, (48,) * dim, 1e-6, 100, [body])
+
+
+# x, T: 0.8 and 2.3 M values in all, i.e. one and three chunks of 2^20
+SIZES = (1, 7, 4096, 33, 200_000, 27_001, 2, 25_000)
+
+
+@pytest.mark.parametrize("dim,mode", [(3, "fp64"), (3, "mixed"), (2, "fp64")])
+def test_many_jobs_equal_each_job(dim, mode):
+    batch = GPUBatch(dim=dim, mode=mode)
+    ids = [batch.add(_cloud(dim, n, 100 + n)) for n in SIZES]
+    batch.step(3)
+    order = ids[::-1] + ids[2:4]    # any order, and a job twice
+    for f in GENERAL:
+        alone = {j: batch.points(j, 0, f) for j in ids}
+        for threads in (1, 3, 64):
+            for got, j in zip(batch.points_many(order, 0, f, threads=threads), order):
+                assert bits_equal(got, alone[j]), f"{f}, {threads} threads, job {j}"
+    assert batch.points_many([], 0, "x") == []
+    batch.close()
