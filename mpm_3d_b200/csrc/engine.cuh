@@ -21,8 +21,8 @@
 #pragma once
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
+#include <condition_variable>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -994,6 +994,14 @@ class Batch : public BatchBase {
     return st;
   }
 
+  // Host threads that copy `total` doubles out: one per 2 MB, as many as asked
+  // for and the host has, and at most 8, beyond which they only wait for one
+  // another (three fields of 8 jobs, 0.66 M points, on 16 cores: 8.2 ms with 8
+  // threads, 13 ms with 16).
+  static int deliver_threads(int64_t total, int asked) {
+    return (int)std::max<int64_t>(1, std::min<int64_t>(std::min(asked, host_threads()), total >> 18));
+  }
+
   // Copies `total` doubles of device memory to consecutive host segments:
   // through two pinned buffers, the next chunk under way while up to
   // `threads` host threads copy the last one out (writing freshly mapped
@@ -1038,21 +1046,28 @@ class Batch : public BatchBase {
       const int64_t a = c * chunk, n = std::min(chunk, total - a);
       copy_out(c, a + n * t / nt, a + n * (t + 1) / nt);
     };
-    // ready: chunks that have arrived; finished: slices copied out; nt: the
-    // threads there are, this one included (set before the first chunk is
-    // announced; fewer than asked for if the system has no more)
-    std::atomic<int64_t> ready{0}, finished{0};
+    // ready: chunks that have arrived (-1: the copies failed); finished: slices
+    // copied out by the other threads; nt: the threads there are, this one
+    // included (set before the first chunk is announced; fewer than asked for if
+    // the system has no more)
+    std::mutex m;
+    std::condition_variable arrived, copied;
+    int64_t ready = 0, finished = 0;
     int nt = 1;
     std::vector<std::thread> pool;
-    const int want = total >= ((int64_t)1 << 18) ? std::max(1, threads) : 1;
+    const int want = deliver_threads(total, threads);
     auto start = [&](int t) {
       pool.emplace_back([&, t]() {
         for (int64_t c = 0; c < chunks; c++) {
-          int64_t r;
-          while ((r = ready.load(std::memory_order_acquire)) <= c && r >= 0) std::this_thread::yield();
-          if (r < 0) return;   // the copies failed
+          {
+            std::unique_lock<std::mutex> lock(m);
+            arrived.wait(lock, [&] { return ready > c || ready < 0; });
+            if (ready < 0) return;
+          }
           slice(c, t, nt);
-          finished.fetch_add(1, std::memory_order_release);
+          std::lock_guard<std::mutex> lock(m);
+          finished++;
+          copied.notify_one();
         }
       });
     };
@@ -1061,18 +1076,24 @@ class Batch : public BatchBase {
     } catch (const std::exception&) {
     }
     nt = 1 + (int)pool.size();
+    auto announce = [&](int64_t r) {
+      std::lock_guard<std::mutex> lock(m);
+      ready = r;
+      arrived.notify_all();
+    };
     cudaError_t e = cudaSuccess;
     for (int64_t c = 0; c < chunks; c++) {
       if (c > 0) e = cudaEventSynchronize(dl_ev_[c & 1]);
       // the other buffer was copied out in the last round
       if (e == cudaSuccess && c + 1 < chunks) e = queue(c + 1);
       if (e != cudaSuccess) {
-        ready.store(-1, std::memory_order_release);
+        announce(-1);
         break;
       }
-      ready.store(c + 1, std::memory_order_release);
+      announce(c + 1);
       slice(c, 0, nt);
-      while (finished.load(std::memory_order_acquire) < (c + 1) * (nt - 1)) std::this_thread::yield();
+      std::unique_lock<std::mutex> lock(m);
+      copied.wait(lock, [&] { return finished == (c + 1) * (nt - 1); });
     }
     for (auto& th : pool) th.join();
     MPM_CUDA_TRY(e);

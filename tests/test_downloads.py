@@ -45,3 +45,28 @@ def test_many_jobs_equal_each_job(dim, mode):
                 assert bits_equal(got, alone[j]), f"{f}, {threads} threads, job {j}"
     assert batch.points_many([], 0, "x") == []
     batch.close()
+
+
+def test_download_threads_are_bounded():
+    """However many threads a caller asks for, at most 8 copy a field out (the
+    caller's own is one of them)."""
+    batch = GPUBatch(dim=3, mode="fp64")
+    job = batch.add(_cloud(3, 600_000, 1))
+    batch.step(1)
+    batch.synchronize()
+    tasks = lambda: len(os.listdir("/proc/self/task"))
+    seen, stop = [], threading.Event()
+
+    def watch():
+        while not stop.is_set():
+            seen.append(tasks())
+
+    watcher = threading.Thread(target=watch)
+    watcher.start()
+    before = tasks()
+    for _ in range(3):
+        batch.points_many([job], 0, "T", threads=64)
+    stop.set()
+    watcher.join()
+    batch.close()
+    assert max(seen) <= before + 7, f"{max(seen) - before} threads beside the caller"
