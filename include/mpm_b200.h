@@ -402,10 +402,21 @@ mpmgpu_status mpmgpu_batch_sizes(const mpmgpu_batch* b, int job, int body, int64
 mpmgpu_status mpmgpu_batch_download_points(mpmgpu_batch* b, int job, int body, int field, double* out);
 /* No counterpart in the reference. One point field of body `body` of each
  * of `count` jobs, outs[k] receiving jobs[k]'s (layout of
- * mpmgpu_download_points): the copies are queued together with one wait and
- * converted to the reference's order on up to `threads` host threads. */
+ * mpmgpu_download_points): converted to the reference's layout and order on
+ * the device, in groups of up to 192 MB (or one body), and copied out of
+ * pinned memory by up to `threads` host threads (at most 8, one per 2 MB).
+ * Without device memory for a group the host converts, one job per thread.
+ * MPMGPU_ERR_UNSUPPORTED while the batch's stream is being captured (the call
+ * waits for its copies); the capture stays valid. Both hold for
+ * mpmgpu_download_points and mpmgpu_batch_download_points too. */
 mpmgpu_status mpmgpu_batch_download_points_many(mpmgpu_batch* b, int count, const int* jobs, int body, int field,
                                                 double* const* outs, int threads);
+
+/* No counterpart in the reference. Device bytes the batch's point downloads
+ * may take for a converted copy, which is not part of any footprint (negative:
+ * the default, a group as above); a download with a larger body is converted
+ * on the host. */
+mpmgpu_status mpmgpu_batch_set_download_limit(mpmgpu_batch* b, int64_t bytes);
 
 /* Frees the job's device memory; it leaves the batch at the next step. */
 mpmgpu_status mpmgpu_batch_remove_job(mpmgpu_batch* b, int job);

@@ -420,6 +420,12 @@ mpmgpu_status mpmgpu_batch_download_points_many(mpmgpu_batch* b, int count, cons
   return b->b->download_points_many(count, jobs, body, field, outs, threads);
 }
 
+mpmgpu_status mpmgpu_batch_set_download_limit(mpmgpu_batch* b, int64_t bytes) {
+  if (!b) return MPMGPU_ERR_ARG;
+  b->b->set_download_limit(bytes);
+  return MPMGPU_OK;
+}
+
 mpmgpu_status mpmgpu_batch_remove_job(mpmgpu_batch* b, int job) {
   if (!b) return MPMGPU_ERR_ARG;
   return b->b->remove_job(job);

@@ -321,8 +321,8 @@ class BatchBase {
   virtual mpmgpu_status remove_job(int job) = 0;
   virtual mpmgpu_status job_state(int job, int64_t* done, int64_t* left) const = 0;
   virtual mpmgpu_status download_points(int job, int body, int field, double* out) = 0;
-  // One point field of one body of each of `count` jobs, copied with one
-  // wait and converted on up to `threads` host threads.
+  // One point field of one body of each of `count` jobs, converted on the
+  // device and copied out by up to `threads` host threads.
   virtual mpmgpu_status download_points_many(int count, const int* jobs, int body, int field, double* const* outs,
                                              int threads) = 0;
   // Raw point state of a body copied to host memory in stream order, i.e.
@@ -355,6 +355,9 @@ class BatchBase {
   // Poll limit of the fused kernels' waits for bulk copies (kWaitPolls by
   // default); a wait that runs out makes the step report MPMGPU_ERR_DEVICE.
   virtual void set_wait_limit(uint32_t polls) = 0;
+  // Device bytes a point download may take for its converted copy (negative:
+  // no limit); what does not fit is converted on the host.
+  virtual void set_download_limit(int64_t bytes) = 0;
   virtual int64_t memory_in_use() const = 0;
   virtual void counts(int* live_jobs, int64_t* live_points) const = 0;
   virtual int points_per_item() const = 0;
@@ -951,21 +954,20 @@ class Batch : public BatchBase {
   // One field of several bodies converted to the reference layout on the
   // device (k_points_field), in groups of at most kFetchGroupBytes (or one
   // body), and delivered to the host arrays. *done = false: nothing was
-  // done, because there is no memory for the converted copy or the stream is
-  // being captured; the caller then converts on the host.
+  // done, because there is no memory for the converted copy or a body's is
+  // beyond the limit set for it; the caller then converts on the host.
   mpmgpu_status download_converted(const std::vector<std::pair<HBody*, double*>>& bodies, int field, int threads,
                                    bool* done) {
     *done = false;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream_, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return MPMGPU_OK;
     const int64_t w = field_width(field);
+    const int64_t most = download_limit_ < 0 ? (int64_t)kFetchGroupBytes : download_limit_;
     int64_t group = 1;
     for (size_t b = 0; b < bodies.size();) {
       int64_t sum = bodies[b].first->n * w;
-      for (b++; b < bodies.size() && (sum + bodies[b].first->n * w) * 8 <= (int64_t)kFetchGroupBytes; b++)
-        sum += bodies[b].first->n * w;
+      for (b++; b < bodies.size() && (sum + bodies[b].first->n * w) * 8 <= most; b++) sum += bodies[b].first->n * w;
       group = std::max(group, sum);
     }
+    if (download_limit_ >= 0 && group * 8 > download_limit_) return MPMGPU_OK;
     double* dev = nullptr;
     if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&dev), (size_t)group * sizeof(double), pool_, stream_) !=
         cudaSuccess) {
@@ -1101,41 +1103,27 @@ class Batch : public BatchBase {
   }
 
   mpmgpu_status download_points(int job, int body, int field, double* out) override {
-    HJob* j;
-    HBody* B;
-    MPM_TRY(readable_body(job, body, &j, &B));
-    const int64_t n = B->n;
-    if (field == MPMGPU_P_B) {
-      MPM_TRY(synchronize());
-      for (int64_t i = 0; i < n; i++)
-        for (int d = 0; d < 3; d++) out[3 * i + d] = j->sp.grav[d];
-      return MPMGPU_OK;
-    }
-    MPM_TRY(point_field_check(*B, field));
-    bool done = false;
-    MPM_TRY(download_converted({{B, out}}, field, host_threads(), &done));
-    if (done) return MPMGPU_OK;
-    // the point ids and the arrays of the field, copied with one wait
-    PointView pv;
-    pv.n = n;
-    std::vector<std::pair<const void*, size_t>> items;
-    std::vector<const void**> slots;
-    point_field_arrays(*B, field, pv, [&](const void* src, size_t bytes, const void** slot) {
-      items.emplace_back(src, bytes);
-      slots.push_back(slot);
-    });
-    std::vector<const unsigned char*> h;
-    MPM_TRY(fetch(items, h));
-    for (size_t k = 0; k < slots.size(); k++) *slots[k] = h[k];
-    points_to_ref(pv, field, out);
-    return MPMGPU_OK;
+    return download_points_many(1, &job, body, field, &out, host_threads());
   }
 
   mpmgpu_status download_points_many(int count, const int* jobs, int body, int field, double* const* outs,
                                      int threads) override {
     if (count < 0 || (count > 0 && (!jobs || !outs))) return fail(MPMGPU_ERR_ARG, "job list missing");
+    // the call waits for its copies, which a stream under capture cannot do;
+    // refused before anything is queued, so the caller's capture stays valid
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    MPM_CUDA_TRY(cudaStreamIsCapturing(stream_, &capture));
+    if (capture != cudaStreamCaptureStatusNone)
+      return fail(MPMGPU_ERR_UNSUPPORTED, "a download waits for its copies and cannot run while the stream is captured");
     if (field == MPMGPU_P_B) {
-      for (int k = 0; k < count; k++) MPM_TRY(download_points(jobs[k], body, field, outs[k]));
+      MPM_TRY(synchronize());
+      for (int k = 0; k < count; k++) {
+        HJob* j;
+        HBody* B;
+        MPM_TRY(readable_body(jobs[k], body, &j, &B));
+        for (int64_t i = 0; i < B->n; i++)
+          for (int d = 0; d < 3; d++) outs[k][3 * i + d] = j->sp.grav[d];
+      }
       return MPMGPU_OK;
     }
     std::vector<std::pair<HBody*, double*>> bodies;
@@ -1199,6 +1187,9 @@ class Batch : public BatchBase {
     return MPMGPU_OK;
   }
   static constexpr size_t kFetchGroupBytes = (size_t)192 << 20;
+
+  void set_download_limit(int64_t bytes) override { download_limit_ = bytes; }
+  int64_t download_limit_ = -1;   // device bytes of a converted copy (-1: none set)
 
   // ---- frames ----
 

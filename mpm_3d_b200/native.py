@@ -137,6 +137,7 @@ def load() -> ctypes.CDLL:
     lib.mpmgpu_batch_job_state.argtypes = [vp, ctypes.c_int, i64p, i64p]
     lib.mpmgpu_batch_sizes.argtypes = [vp, ctypes.c_int, ctypes.c_int, i64p, i64p]
     lib.mpmgpu_batch_download_points.argtypes = [vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, vp]
+    lib.mpmgpu_batch_set_download_limit.argtypes = [vp, ctypes.c_int64]
     lib.mpmgpu_batch_download_points_many.argtypes = [vp, ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.c_int,
                                                       ctypes.c_int, ctypes.POINTER(ctypes.c_void_p), ctypes.c_int]
     lib.mpmgpu_batch_remove_job.argtypes = [vp, ctypes.c_int]
@@ -504,8 +505,8 @@ class GPUBatch:
         return out
 
     def points_many(self, jobs, b: int, name: str, threads: int = 0):
-        """One point field of body b of several jobs, copied with one wait
-        and converted on host threads (all host threads by default)."""
+        """One point field of body b of several jobs, converted on the device
+        and copied out on host threads (by default as many as pay)."""
         fid, w = POINT_FIELDS[name]
         outs = [np.zeros((self.cases[j].bodies[b].n, w)) for j in jobs]
         ids = (ctypes.c_int * len(jobs))(*jobs)
@@ -513,6 +514,11 @@ class GPUBatch:
         self._check(self.lib.mpmgpu_batch_download_points_many(self.h, len(jobs), ids, b, fid, ptrs,
                                                                threads or (os.cpu_count() or 1)))
         return outs
+
+    def set_download_limit(self, nbytes: int):
+        """Device bytes a download may take for its converted copy (-1: the
+        default); a download with a larger body is converted on the host."""
+        self._check(self.lib.mpmgpu_batch_set_download_limit(self.h, nbytes))
 
     def remove(self, job: int):
         self._check(self.lib.mpmgpu_batch_remove_job(self.h, job))

@@ -44,7 +44,55 @@ def test_many_jobs_equal_each_job(dim, mode):
             for got, j in zip(batch.points_many(order, 0, f, threads=threads), order):
                 assert bits_equal(got, alone[j]), f"{f}, {threads} threads, job {j}"
     assert batch.points_many([], 0, "x") == []
+    # the same in groups of one or a few jobs, and converted on the host: with
+    # 16 MB each job fits and all together do not, with 1 MB the largest does
+    # not, and with 0 none does
+    for limit in (16 << 20, 1 << 20, 0):
+        for f in GENERAL:
+            alone = {j: batch.points(j, 0, f) for j in ids}
+            batch.set_download_limit(limit)
+            for threads in (1, 3):
+                for got, j in zip(batch.points_many(order, 0, f, threads=threads), order):
+                    assert bits_equal(got, alone[j]), f"{f}, limit {limit}, {threads} threads, job {j}"
+            for j in ids:
+                assert bits_equal(batch.points(j, 0, f), alone[j]), f"{f}, limit {limit}, job {j} alone"
+            batch.set_download_limit(-1)
     batch.close()
+
+
+def test_fields_of_debug_and_granular_bodies():
+    batch = GPUBatch(dim=3, mode="fp64", keep_debug=True)
+    sand = inputs.sand_column(3, n_cells=12, steps=30)
+    job = batch.add(sand)
+    batch.step(20)
+    for f in ("L", "gammap", "gammap_dot", "T"):
+        device = batch.points(job, 0, f)
+        assert np.abs(device).max() > 0.0
+        batch.set_download_limit(0)
+        assert bits_equal(batch.points(job, 0, f), device), f
+        batch.set_download_limit(-1)
+    batch.close()
+
+
+def test_download_is_refused_while_the_stream_is_captured():
+    """The call waits for its copies, so a captured stream cannot serve it: an
+    error, nothing queued, and the capture stays valid."""
+    torch = pytest.importorskip("torch")
+    sim = GPUExplicitUSL(inputs.two_body_collision_3d(16, steps=2, gap=0.01))
+    sim.step(1)
+    want = sim.points(0, "x")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(torch.cuda.ExternalStream(sim.stream())):
+        graph.capture_begin()
+        try:
+            for f in ("x", "T", "b"):
+                with pytest.raises(MpmGpuError, match="captured"):
+                    sim.points(0, f)
+        finally:
+            graph.capture_end()
+    del graph
+    assert bits_equal(sim.points(0, "x"), want)
+    sim.close()
 
 
 def test_download_threads_are_bounded():
