@@ -1521,6 +1521,7 @@ class Batch : public BatchBase {
     MPM_TRY(commit());
     if (live_jobs_ == 0) return fail(MPMGPU_ERR_STATE, "no jobs to tune on");
     MPM_TRY(snapshot_save());
+    const bool cap_auto = cap_auto_, sort_auto = sort_auto_;
     cap_auto_ = sort_auto_ = false;   // from here on the tuner's choices
     const int original_cap = cap_, original_si = sort_interval_;
     cudaEvent_t e0, e1;
@@ -1583,6 +1584,13 @@ class Batch : public BatchBase {
     cap_ = (st == MPMGPU_OK) ? best_c : original_cap;
     form_ = (st == MPMGPU_OK) ? best_f : original_form;
     sort_interval_ = (st == MPMGPU_OK) ? best_si : original_si;
+    if (st != MPMGPU_OK) {
+      // nothing was chosen: the defaults hold again, and the next step re-bins
+      // (the work list is that of the failed trial's item size)
+      cap_auto_ = cap_auto;
+      sort_auto_ = sort_auto;
+      membership_dirty_ = true;
+    }
     drop_graphs();
     snapshot_free();
     MPM_TRY(st);
