@@ -2391,6 +2391,13 @@ class Batch : public BatchBase {
   }
 
   mpmgpu_status launch_step_direct() {
+    // a launch that failed after the last grid update left its counts standing
+    // (the fused launch closes them): the block list must start from zero
+    if (publish_) {
+      MPM_CUDA_TRY(cudaMemsetAsync(count_, 0, sizeof(unsigned long long), stream_));
+      MPM_CUDA_TRY(cudaMemsetAsync(active_acc_, 0, sizeof(unsigned long long), stream_));
+    }
+    publish_ = true;   // until the step's first fused launch closes this grid update's counts
     if (hdr_host_.blocks <= kScanBlocks) {
       StageTimer timer(this, kStageGrid);
       const int gb = (int)std::max<int64_t>(1, std::min<int64_t>(sm_count_ * 8, (hdr_host_.blocks + 3) / 4));
@@ -2416,7 +2423,6 @@ class Batch : public BatchBase {
         k_grid<2><<<gb, 64, 0, stream_>>>(insts_d_, gbodies_d_, blk_inst_, list_, count_, active_acc_);
       MPM_TRY(check_launch("k_grid"));
     }
-    publish_ = true;   // the step's first fused launch closes the grid update's counts
     if (det_) {
       // update, bounds from the new state, then the scatter
       MPM_TRY(launch_fused(0, 1));
