@@ -9,7 +9,7 @@ import pytest
 
 import bridge
 from mpm_3d_b200 import inputs
-from mpm_3d_b200.native import GPUExplicitUSL
+from mpm_3d_b200.native import GPUBatch, GPUExplicitUSL
 from util import FP64_TOL, assert_close, field_floor
 
 pytestmark = pytest.mark.gpu
@@ -93,6 +93,76 @@ def test_cell_sums_mixed(name, kernel):
     ref.step(6)
     for f in ("x", "x_t", "T"):
         assert_close(gpu.points(0, f), ref.points(0, f), 1e-4, f"{name} {f}", field_floor(case, f))
+    gpu.close()
+
+
+# The same clouds as the first body of a contact (contact normals, the second
+# body close by or out of reach) and, over the body table, as jobs of a batch of
+# seven bodies with and without contact: the items of one kind are passed over
+# by the other kind's launch, and tiles are loaded ahead across bodies.
+def _with_contact(name):
+    case = CLOUDS[name]()
+    rng = np.random.default_rng(31)
+    x = np.clip(case.bodies[0].x[:64] + rng.uniform(-0.4, 0.4, (min(64, case.bodies[0].n), 3)) * H, 0.05, 0.95)
+    n, vol = len(x), (H / 2) ** 3
+    other = inputs.Body("other", np.full(n, 1000.0 * vol), np.full(n, vol), x, -case.bodies[0].x_t[:n],
+                        np.ones(n, np.int32), E=1e4)
+    case.bodies.append(other)
+    case.contacts.append(inputs.Contact(0, 1, 0.3))
+    return case
+
+
+# "one_point" is left out: a lone pair's contact normal divides two sums of
+# rounding size, which no two orders agree on
+@pytest.mark.parametrize("cap", [128, 512])
+@pytest.mark.parametrize("name", sorted(set(CLOUDS) - {"one_point"}))
+def test_cell_sums_in_contact_and_over_the_table(name, cap):
+    both, alone = _with_contact(name), CLOUDS[name]()
+    cases = [both, alone, both, CLOUDS["drift_down"](), alone]
+    batch = GPUBatch(dim=3, mode="fp64", kernel=("point_per_thread", cap))
+    ids = [batch.add(c, steps=4) for c in cases]
+    solo = GPUExplicitUSL(both, kernel=("point_per_thread", cap))
+    refs = {id(c): bridge.RestatedJob(c) for c in (both, alone, cases[3])}
+    batch.step(4)
+    solo.step(4)
+    for ref in refs.values():
+        ref.step(4)
+    for f in ("x", "x_t", "T", "v"):
+        for b in range(2):
+            assert_close(solo.points(b, f), refs[id(both)].points(b, f), 4 * FP64_TOL, f"{name} contact body {b} {f}",
+                         field_floor(both, f))
+        for j, c in zip(ids, cases):
+            for b in range(len(c.bodies)):
+                assert_close(batch.points(j, b, f), refs[id(c)].points(b, f), 4 * FP64_TOL, f"{name} job {j} body {b} {f}",
+                             field_floor(c, f))
+    solo.close()
+    batch.close()
+
+
+# Both grid updates: from the flags (up to 16,384 node blocks) and from the list
+# of active blocks (above), in 2D (blocks of 8 x 8 nodes) and 3D (4 x 4 x 4).
+@pytest.mark.parametrize("dim,n", [(2, 1016), (2, 1040), (3, 96), (3, 104)])
+def test_grid_update_on_either_side_of_the_block_limit(dim, n):
+    h = 1.0 / n
+    rng = np.random.default_rng(41)
+    x, v = np.zeros((3000, 3)), np.zeros((3000, 3))
+    x[:, :dim] = 0.5 + rng.uniform(-12, 12, (3000, dim)) * h
+    v[:, :dim] = rng.uniform(-1.0, 1.0, (3000, dim))
+    vol = (h / 2) ** dim
+    body = inputs.Body("cloud", np.full(3000, 1000.0 * vol), np.full(3000, vol), x, v, np.ones(3000, np.int32), E=1e4)
+    case = inputs.Case("cloud", dim, (1.0,) * dim, (n,) * dim, 1e-6, 4, [body])
+    blocks = ((n + 1 + 7) // 8) ** 2 if dim == 2 else ((n + 1 + 3) // 4) ** 3
+    assert (blocks <= 16384) == (n in (1016, 96))
+    gpu = GPUExplicitUSL(case, keep_debug=True)
+    ref = bridge.RestatedJob(case)
+    for s in range(4):
+        gpu.step(1)
+        ref.step(1)
+        for f in ("x", "x_t", "T", "v"):
+            assert_close(gpu.points(0, f), ref.points(0, f), (s + 1) * FP64_TOL, f"step {s} {f}", field_floor(case, f))
+    m = ref.nodes(0, "m")
+    assert_close(gpu.nodes(0, "m"), m, FP64_TOL, "nodal m")
+    assert gpu.active_nodes()[0] == int((m > 0).sum())
     gpu.close()
 
 

@@ -51,6 +51,33 @@ def test_wait_that_runs_out_is_reported_and_contained():
     sim.close()
 
 
+@pytest.mark.parametrize("bodies", [1, 5])
+def test_wait_of_the_point_per_thread_kernel_that_runs_out(bodies):
+    """The same in 3D: launched body by body, where the point arrays arrive by
+    bulk copies, and over the body table, whose entries do too."""
+    bridge.build_restated()
+    case = inputs.column_collapse_3d(scale=16, steps=8)
+    case.bodies = case.bodies * bodies
+    sim = GPUExplicitUSL(case)
+    sim.step(3)
+    sim.synchronize()
+    sim.set_wait_limit(0)
+    sim.step(1)
+    with pytest.raises(MpmGpuError, match="wait limit"):
+        sim.synchronize()
+    sim.close()
+    sim = GPUExplicitUSL(case)
+    ref = bridge.RestatedJob(case)
+    sim.step(5)
+    ref.step(5)
+    sim.synchronize()
+    for b in range(bodies):
+        for f in FIELDS:
+            assert_close(sim.points(b, f), ref.points(b, f), 5 * FP64_TOL, f"after a timed-out handle: {f}",
+                         field_floor(case, f))
+    sim.close()
+
+
 def test_request_larger_than_the_budget_is_rejected_at_submission():
     case = inputs.serving_case(inputs.serving_stream(rate=50.0, duration=0.2, seed=5, n_range=(16, 16),
                                                      steps_range=(10, 10))[0])

@@ -29,6 +29,13 @@ def _cpdi_off_2d():
     return c
 
 
+def _cpdi_off_3d():
+    c = inputs.two_body_collision_3d(16, steps=15, gap=0.01)
+    c.cpdi = 0
+    c.name += "_cpdi_off"
+    return c
+
+
 def _explicit_contact_3d():
     c = inputs.two_body_collision_3d(16, steps=10, gap=0.01)
     c.contact_spec = 0
@@ -105,6 +112,7 @@ CASES = {
     "block_drop_2d": (inputs.block_drop_2d, 120),
     "spinning_block_2d": (_spinning_block_2d, 120),
     "block_drop_2d_cpdi_off": (_cpdi_off_2d, 40),
+    "collision_3d_cpdi_off": (_cpdi_off_3d, 15),
     "collision_2d": (lambda: inputs.two_body_collision_2d(20, steps=60), 60),
     "collision_3d_touching": (lambda: inputs.two_body_collision_3d(16, steps=15, gap=0.01), 15),
     "collision_3d_explicit": (_explicit_contact_3d, 8),
@@ -169,15 +177,15 @@ def test_step_parity(name):
 
 
 CASES_3D = sorted(n for n in CASES if "3d" in n)
-KERNEL_FORMS = [("staged", 512), ("staged", 256), ("point_per_thread", 128), ("point_per_thread", 256)]
+KERNEL_FORMS = [("staged", 512), ("staged", 256), ("point_per_thread", 128), ("point_per_thread", 256),
+                ("point_per_thread", 512)]
 
 
 @pytest.mark.parametrize("kernel", KERNEL_FORMS, ids=lambda k: f"{k[0]}{k[1]}")
 @pytest.mark.parametrize("name", CASES_3D)
 def test_step_parity_kernel_forms(name, kernel):
-    """3D jobs run on the one-point-per-thread kernel with 512 points per
-    item by default (test_step_parity); every other kernel form and size
-    must meet the same parity."""
+    """Every kernel form and size meets the parity, whichever the default
+    takes for a job of this size (test_step_parity)."""
     _step_parity(name, kernel=kernel)
 
 
