@@ -338,19 +338,9 @@ __device__ __forceinline__ int build_map(const Geom& g, const MapConst& mc, int 
   return build_map_fast<DIM>(g, mc, cpdi, x, ext, pm, err, map_grad_scale(g, ext));
 }
 template <int DIM>
-__device__ __forceinline__ int build_map(const Geom& g, const MapConst& mc, int cpdi, const double* x, double ext,
-                                         PointMapT<double>& pm, int* err, double sG) {
-  return build_map_fast<DIM>(g, mc, cpdi, x, ext, pm, err, sG);
-}
-template <int DIM>
 __device__ __forceinline__ int build_map(const Geom& g, const MapConst& mc, int cpdi, const double* x, float ext,
                                          PointMapT<float>& pm, int* err) {
   return build_map_f32<DIM>(g, mc, cpdi, x, ext, pm, err, map_grad_scale(g, ext));
-}
-template <int DIM>
-__device__ __forceinline__ int build_map(const Geom& g, const MapConst& mc, int cpdi, const double* x, float ext,
-                                         PointMapT<float>& pm, int* err, float sG) {
-  return build_map_f32<DIM>(g, mc, cpdi, x, ext, pm, err, sG);
 }
 
 }  // namespace mpmb200
