@@ -149,7 +149,9 @@ inline bool cap_available(int dim, bool mixed, int cap) {
 // and the time of a step is that of one item. Measured (us per step, 512 ->
 // 128): 1,728 points 27.8 -> 23.1, 43,904 sand points 28.4 -> 24.1, two
 // bodies of 27,000 points 35.6 -> 32.9, of 32,768 points 37.6 -> 36.5; column
-// of 96,000 points 28.5 -> 32.7, 128,000 sand points 32.8 -> 40.6.
+// of 96,000 points 28.5 -> 32.7, 128,000 sand points 32.8 -> 40.6. Launches over
+// the body table: eight jobs of 13,824 points in all 35.2 -> 32.9 (mixed 34.5 ->
+// 34.8), of 46,656 points 50.2 -> 41.3 (48.9 -> 42.5).
 constexpr int64_t kSmallPoints = 65536;
 
 // Above that they follow the points of a filled bin (64 cells), estimated from
@@ -171,7 +173,8 @@ inline int items_for_bin(double points_per_bin) { return points_per_bin <= 1.02 
 // in 2.6 M points 3.4 % of the visits at an interval of 32, 0.4 % at 16 (727
 // -> 681 us per step; 692 at 20, 668 at 12, 678 at 8; mixed, 0.5 M points:
 // 179 -> 173, 176 at 12). Bodies that hardly drift pay for the re-binning
-// alone: column 384 us at 32, 395 at 16.
+// alone: column 384 us at 32, 395 at 16; eight small jobs in 2D or 3D 2 to 4 %
+// (1,152 points in all 25.6 -> 26.3 us per step).
 constexpr int kSortInterval = 32, kSortIntervalTable = 16;
 
 // Forms of the fused kernel (mpmgpu_set_kernel): the staged kernel

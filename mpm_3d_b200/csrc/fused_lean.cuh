@@ -6,12 +6,12 @@
 // A CTA of NT threads works on one work item at a time (at most PPT * NT
 // points of one bin of one body, PPT points per thread):
 //   0. the CTA stages the nodal velocities of the bin's node tile;
-//   1. each thread takes its points (global loads, coalesced: consecutive
-//      threads, consecutive points) through gather, state update (movePoints,
+//   1. each thread takes its points (their arrays staged in shared memory by
+//      bulk copies) through gather, state update (movePoints,
 //      calculateStrainRate, updateDensity, updateStress) and map build at the
 //      new position, writes what the scatter needs of the point (a record: two
-//      numbers per axis and the 10 scatter sources) to shared memory and links
-//      it into the list of its window's base cell;
+//      numbers per axis and the 10 scatter sources) over its staged state and
+//      links it into the list of its window's base cell;
 //   2. four threads per non-empty cell, one per node row (y, z offset 0 or 1)
 //      of the cell's window, walk the cell's list and accumulate the row's
 //      nodes in registers, then add them into the global accumulators (one
@@ -26,29 +26,31 @@
 // no thread waits for.
 //
 // Measured against the kernel that added every point's contributions to a
-// shared tile (us per step): column collapse of 3.1 M points 499 -> 383
-// (291 algorithmic bytes per point: 2.0 -> 2.6 TB/s), two-body collision of
-// 0.52 M points 171 -> 110, 21 block drops of 2.6 M points in all 952 -> 730,
-// 1,728 points 51 -> 31. What bounds it now: 16 warps per SM (128 registers,
-// 110 KB of shared memory per CTA) on chains of FP64 operations of 11 cycles
-// each, at 45 % of the issue slots; FP64 pipe 24 %, shared-memory wavefronts
-// 34 %. Tried and slower: 24 warps at 80 registers with items of 256 points
-// (item costs are paid twice, 472 us on the column), the velocity tile as
-// whole node blocks by bulk copies (the node blocks then straddle the bins,
-// whose adds meet in twice the memory sectors: 4 to 15 %), the rows' sums
-// combined in shared memory before the adds (spills), an L2 prefetch of the
-// next item's arrays (1 %).
+// shared tile (us per step): column collapse of 3.1 M points 499 -> 386 (the
+// kernel alone 468 -> 350, 291 algorithmic bytes per point: 2.0 -> 2.6 TB/s),
+// two-body collision of 0.52 M points 171 -> 108, 21 block drops of 2.6 M points
+// in all 952 -> 657, 1,728 points 51 -> 23. The column's figures are those of
+// its initial lattice, where no window spans three nodes: once half of its
+// points have a wide axis a step takes 600 us (a wide point gathers in rolled
+// loops, and one wide along y or z enters two or four cells' lists). What bounds
+// it now: 16 warps per SM (128 registers, 110 KB of shared memory per CTA) on
+// chains of FP64 operations of 11 cycles each: on the column 42 % of the issue
+// slots, FP64 pipe 31 %, shared-memory wavefronts 42 %. Tried and slower: 24
+// warps at 80 registers with items of 256 points (item costs are paid twice, 472
+// us on the column), the velocity tile as whole node blocks by bulk copies (the
+// node blocks then straddle the bins, whose adds meet in twice the memory
+// sectors: 4 to 15 %), the rows' sums combined in shared memory before the adds
+// (spills), an L2 prefetch of the next item's arrays (1 %).
 #pragma once
 
 #include "fused.cuh"
 
 namespace mpmb200 {
 
-// Points per work item the autotuner chooses from: 128 (CTAs of 128
-// threads), 256 (256 threads) and 512 (256 threads, two points each: one
-// tile load and one set of nodal adds for a whole 4x4x4 bin of 8 points per
-// cell). 512 is the default: 10 to 40 % ahead of 256 and 128 from about
-// 50,000 points on.
+// Points per work item: 128 (CTAs of 128 threads), 256 (256 threads) or 512 (256
+// threads, two points each: one tile load and one set of nodal adds for a whole
+// 4x4x4 bin of 8 points per cell). The engine's defaults choose between 128 and
+// 512 (kSmallPoints, items_for_bin); 256 is for the autotuner and the caller.
 __host__ __device__ constexpr bool lean_size_ok(int cap) { return cap == 128 || cap == 256 || cap == 512; }
 constexpr int kDefaultLeanCap = 512;
 
@@ -553,6 +555,8 @@ __device__ __forceinline__ void lean_point(const BodyCtx<PT>& c, int* err, int64
         lean_far_push(sh, j, kFarPoint);
         return;
       }
+      // over the lanes that are here together: each of them gets the mask that
+      // names them all, and any such set gives a lane loops that cover its own bits
       const int any = __reduce_or_sync(__activemask(), lm.fl & 7);
       gs = any == 0 ? lean_gather<T, TN, false>(lm, o, tvel, 0) : lean_gather<T, TN, true>(lm, o, tvel, any);
       if constexpr (sizeof(PT) == 4) {
