@@ -84,8 +84,8 @@ ENSEMBLE_SEED = 1003
 # captures of the kernel (the ensemble's from a capture of its first 96 jobs,
 # scaled to a launch by its points; the column's at full size). None where no
 # capture exists.
-TRAFFIC_BYTES_PER_POINT = {("ensemble", "mixed"): 218.4, ("ensemble", "fp64"): 305.5, ("column", "fp64"): 307.1,
-                           ("column", "mixed"): 212.9}
+TRAFFIC_BYTES_PER_POINT = {("ensemble", "mixed"): 220.9, ("ensemble", "fp64"): 305.9, ("column", "fp64"): 310.0,
+                           ("column", "mixed"): 214.0}
 
 
 def make_workload(name: str, rank: int = 0):

@@ -27,15 +27,15 @@
 //
 // Measured against the kernel that added every point's contributions to a
 // shared tile (us per step): column collapse of 3.1 M points 499 -> 386 (the
-// kernel alone 468 -> 350, 291 algorithmic bytes per point: 2.0 -> 2.6 TB/s),
+// kernel alone 468 -> 359, 291 algorithmic bytes per point: 2.0 -> 2.5 TB/s),
 // two-body collision of 0.52 M points 171 -> 108, 21 block drops of 2.6 M points
 // in all 952 -> 657, 1,728 points 51 -> 23. The column's figures are those of
 // its initial lattice, where no window spans three nodes: once half of its
 // points have a wide axis a step takes 600 us (a wide point gathers in rolled
 // loops, and one wide along y or z enters two or four cells' lists). What bounds
 // it now: 16 warps per SM (128 registers, 110 KB of shared memory per CTA) on
-// chains of FP64 operations of 11 cycles each: on the column 42 % of the issue
-// slots, FP64 pipe 31 %, shared-memory wavefronts 42 %. Tried and slower: 24
+// chains of FP64 operations of 11 cycles each: on the column 41 % of the issue
+// slots, FP64 pipe 29 %, shared-memory wavefronts 42 %. Tried and slower: 24
 // warps at 80 registers with items of 256 points (item costs are paid twice, 472
 // us on the column), the velocity tile as whole node blocks by bulk copies (the
 // node blocks then straddle the bins, whose adds meet in twice the memory

@@ -1,7 +1,7 @@
 """The deterministic FP64 form (MPMGPU_MODE_FP64_DETERMINISTIC).
 
 Nodal sums are pre-rounded into two levels whose partial sums are exact in
-any order (kernels_fp64.cuh, make_split / presplit), so the result cannot
+any order (material.cuh, make_split / presplit), so the result cannot
 depend on the order of the atomics, on the point storage order (re-binning
 interval) or on the other jobs of a batch: runs are compared bit for bit.
 Against the oracle it meets the FP64 tolerance of the plain form (1e-10).
