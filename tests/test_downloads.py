@@ -111,7 +111,9 @@ def test_download_threads_are_bounded():
 
     watcher = threading.Thread(target=watch)
     watcher.start()
+    batch.points_many([job], 0, "T", threads=1)   # what the first call of a process starts
     before = tasks()
+    seen.clear()
     for _ in range(3):
         batch.points_many([job], 0, "T", threads=64)
     stop.set()
